@@ -30,6 +30,7 @@
 // contraction (-fmad=false), so the plain FP64 form reproduces the reference
 // rounding sequence; only reduction order in the solver differs.
 
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -1080,6 +1081,7 @@ __global__ void __launch_bounds__(kBlock) k_ve_stress(DevProg P, DevFields F)
 // Poisson: divergence rhs + first CG residual
 // ---------------------------------------------------------------------------
 #include "hf_pcg.cuh"
+#include "hf_solve.cuh"
 
 // ---------------------------------------------------------------------------
 // BiCGStab on the same operator (non-symmetric rows, e.g. AMR interfaces)
@@ -1453,6 +1455,18 @@ struct hf_case {
     VLev<float> *h32 = nullptr;
     TailInst<double> *t64 = nullptr;
     TailInst<float> *t32 = nullptr;
+    // one launch per cluster size runs the whole solve of its instances
+    // (hf_solve.cuh) in place of the loop of level-synchronous kernels
+    bool fused = false;
+    struct SolveLaunch {
+        int first, count, cluster, fine, threads;
+        size_t smem;
+    };
+    std::vector<SolveLaunch> solves;
+    SInst<double> *si64 = nullptr;
+    SInst<float> *si32 = nullptr;
+    std::vector<cudaStream_t> solve_streams;   // the launches of one solve run side by side
+    std::vector<cudaEvent_t> solve_events;
     int64_t coarse_rows = 0, coarse_dense = 0;
     std::vector<int64_t> lrows, lnnz_a, lnnz_p, lnnz_r;
     int body_kernels = 0;           // kernels of one loop body (two iterations)
@@ -1884,6 +1898,195 @@ VLev<T> make_level(char *base, const LevelOff &o, const LevelHost &h, const TRow
     return v;
 }
 
+// Instances of up to this many rows are solved by one cluster each
+// (hf_solve.cuh); a case with a larger one runs the level-synchronous kernels,
+// which spread over the whole device.
+constexpr int kSolveMaxRows = 1 << 19;
+
+// The one-launch solves' tables of every instance on the device, the instances
+// grouped by cluster size (one launch each), largest first.
+template <typename T>
+auto solve_kernel(int fine) -> void (*)(PcgFine, SolveArgs<T>)
+{
+    constexpr bool mix = std::is_same<T, float>::value;
+    return fine == 5 ? k_solve<T, mix, 5> : fine == 7 ? k_solve<T, mix, 7> : k_solve<T, mix, 0>;
+}
+
+template <typename T>
+int build_solve(hf_case *C, const std::vector<const solve::HostSolve *> &F, const std::vector<const std::vector<double> *> &inv,
+                SInst<T> *&dev)
+{
+    const int ni = C->ninst;
+    std::vector<int> order(ni);
+    for (int i = 0; i < ni; i++) order[i] = i;
+    auto rows = [&](int i) { return C->coff[i + 1] - C->coff[i]; };
+    auto key = [&](int i) { return F[i]->cluster * 64 + F[i]->fine; };
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
+        if (key(a) != key(b)) return key(a) > key(b);
+        return rows(a) > rows(b);
+    });
+    Arena ar;
+    std::vector<SInst<T>> I(ni);
+    struct Where {
+        size_t tables, rows_r, rows_u, gvec, rng;
+    };
+    std::vector<Where> W(ni);
+    std::vector<size_t> smem(ni, 0);
+    for (int k = 0; k < ni; k++) {
+        const int i = order[k];
+        const solve::HostSolve &f = *F[i];
+        const int C0 = f.cluster;
+        SInst<T> &o = I[k];
+        memset(&o, 0, sizeof o);
+        o.inst = i;
+        o.row0 = C->coff[i];
+        o.n = rows(i);
+        o.s = f.s;
+        o.clev = f.clev;
+        o.nc = f.nc;
+        // shared memory, in this order as far as each piece fits: the tail's
+        // vectors (always), the vectors with halos, the finest vectors' own
+        // rows, row descriptors and operator tables of the finest level, the
+        // tail's, and the levels' between
+        size_t at = 0;
+        auto take = [&](size_t bytes, size_t keep = 0) -> uint32_t {
+            bytes = (bytes + 15) & ~size_t(15);
+            if (at + bytes + keep > kSolveSmem) return kSolveGlobal;
+            const uint32_t r = (uint32_t)at;
+            at += bytes;
+            return r;
+        };
+        auto elems = [&](uint32_t b) { return b == kSolveGlobal ? b : (uint32_t)(b / sizeof(T)); };
+        const int nl = (int)f.L.size();
+        for (int l = std::max(1, f.s); l < f.clev; l++) {
+            o.L[l].vb = elems(take(sizeof(T) * f.L[l].n));
+            o.L[l].vo = elems(take(sizeof(T) * f.L[l].n));
+        }
+        o.cvec = elems(take(sizeof(T) * 2 * f.nc));
+        o.vr = take(sizeof(T) * f.held[0]);
+        o.vz = take(sizeof(T) * f.held[1]);
+        size_t g = 0;
+        for (int l = 1; l < f.s; l++) {
+            o.L[l].vb = elems(take(sizeof(T) * f.held[2 * l]));
+            o.L[l].vo = elems(take(sizeof(T) * f.held[2 * l + 1]));
+            o.L[l].gb = (uint32_t)g;
+            o.L[l].go = (uint32_t)(g + f.L[l].n);
+            g += 2 * (size_t)f.L[l].n;
+        }
+        const size_t own = (o.n + C0 - 1) / C0, reserve = 48 * 1024;
+        o.vq = take(sizeof(T) * own, reserve);
+        o.vp = take(sizeof(T) * own, reserve);
+        o.vx = take((C->mixed ? sizeof(T) : sizeof(double)) * own, reserve);
+        std::vector<uint2> rr;
+        std::vector<uint4> ru;
+        std::vector<char> blob;
+        for (int l = 0; l < nl; l++) {
+            const solve::HostSolve::Level &h = f.L[l];
+            SLevel &v = o.L[l];
+            v.n = h.n;
+            v.lanes_r = h.lanes_r;
+            v.lanes_u = h.lanes_u;
+            v.row_r = (uint32_t)rr.size();
+            v.row_u = (uint32_t)ru.size();
+            rr.insert(rr.end(), h.rows_r.begin(), h.rows_r.end());
+            ru.insert(ru.end(), h.rows_u.begin(), h.rows_u.end());
+        }
+        auto part = [&](const void *data, size_t bytes, size_t keep = 0) {
+            STab t;
+            t.g = (uint32_t)blob.size();
+            t.bytes = (uint32_t)((bytes + 15) & ~size_t(15));
+            t.s = take(bytes, keep);
+            blob.insert(blob.end(), (const char *)data, (const char *)data + bytes);
+            blob.resize((blob.size() + 15) & ~size_t(15), 0);
+            return t;
+        };
+        auto ents = [&](const std::vector<int32_t> &off, const std::vector<double> &val) {
+            std::vector<SEnt<T>> e(off.size());
+            memset(e.data(), 0, e.size() * sizeof(SEnt<T>));
+            for (size_t q = 0; q < e.size(); q++) {
+                e[q].off = off[q];
+                e[q].v = (T)val[q];
+            }
+            return part(e.data(), e.size() * sizeof(SEnt<T>));
+        };
+        auto level_rows = [&](int l) {
+            // own rows of a distributed level, all of a tail level's
+            const size_t nu = f.L[l].n, nr = f.L[l].rows_r.size(), d = l < f.s ? C0 : 1;
+            o.L[l].srow_u = take(sizeof(uint4) * ((nu + d - 1) / d));
+            o.L[l].srow_r = take(sizeof(uint2) * ((nr + d - 1) / d));
+        };
+        auto level_tabs = [&](int l) {
+            o.L[l].m = ents(f.L[l].off_m, f.L[l].v_m);
+            o.L[l].p = ents(f.L[l].off_p, f.L[l].v_p);
+            o.L[l].r = ents(f.L[l].off_r, f.L[l].v_r);
+        };
+        o.a = ents(f.L[0].off_m, f.L[0].v_a);
+        level_tabs(0);
+        level_rows(0);
+        {
+            std::vector<T> d(inv[i]->begin(), inv[i]->end());
+            o.inv = part(d.data(), d.size() * sizeof(T));
+        }
+        for (int l = f.clev - 1; l >= std::max(1, f.s); l--) {
+            level_rows(l);
+            level_tabs(l);
+        }
+        for (int l = f.s - 1; l > 0; l--) {
+            level_rows(l);
+            level_tabs(l);
+        }
+        if (C->mixed) {
+            std::vector<SEnt<double>> e(f.L[0].off_m.size());
+            for (size_t q = 0; q < e.size(); q++) e[q] = SEnt<double>{f.L[0].v_a[q], f.L[0].off_m[q], 0};
+            o.a64 = part(e.data(), e.size() * sizeof(SEnt<double>));
+        }
+        smem[k] = at;
+        W[k] = Where{ar.vec(blob), ar.vec(rr), ar.vec(ru), ar.zeros<T>(g), ar.vec(f.rng)};
+    }
+    char *base = nullptr;
+    HF_CK(cudaMallocAsync((void **)&base, ar.host.size(), C->stream));
+    C->owned.push_back(base);
+    C->bytes += (double)ar.host.size();
+    HF_CK(cudaMemcpyAsync(base, ar.host.data(), ar.host.size(), cudaMemcpyHostToDevice, C->stream));
+    for (int k = 0; k < ni; k++) {
+        I[k].tables = base + W[k].tables;
+        I[k].rows_r = (const uint2 *)(base + W[k].rows_r);
+        I[k].rows_u = (const uint4 *)(base + W[k].rows_u);
+        I[k].gvec = (T *)(base + W[k].gvec);
+        I[k].rng = (const int4 *)(base + W[k].rng);
+    }
+    int rc = upload(C->owned, &dev, I.data(), I.size(), C->bytes, C->stream);
+    if (rc) return rc;
+    HF_CK(cudaStreamSynchronize(C->stream));   // the host copies go away with this function
+    for (int k = 0; k < ni;) {
+        const solve::HostSolve &f = *F[order[k]];
+        int e = k, own = 0;
+        size_t most = 0;
+        for (; e < ni && key(order[e]) == key(order[k]); e++) {
+            most = std::max(most, smem[e]);
+            own = std::max(own, (I[e].n + f.cluster - 1) / f.cluster);
+        }
+        // one row per thread as far as a block goes
+        int threads = std::min(kSolveThreads, std::max(256, (own + 31) / 32 * 32));
+        C->solves.push_back(hf_case::SolveLaunch{k, e - k, f.cluster, f.fine, threads, most});
+        auto *kern = solve_kernel<T>(f.fine);
+        HF_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSolveSmem));
+        HF_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        k = e;
+    }
+    for (size_t k = 1; k < C->solves.size(); k++) {
+        cudaStream_t st = nullptr;
+        HF_CK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+        C->solve_streams.push_back(st);
+    }
+    for (size_t k = 0; k < C->solves.size() && C->solves.size() > 1; k++) {
+        cudaEvent_t ev = nullptr;
+        HF_CK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+        C->solve_events.push_back(ev);
+    }
+    return HF_OK;
+}
+
 // Per-instance smoothed-aggregation hierarchies (hf_amg.cuh), concatenated
 // level by level, the finest-level CG state and the loop control.
 int build_pcg(hf_case *C, const std::vector<int32_t> &mptr, const std::vector<int32_t> &mcol,
@@ -1894,6 +2097,7 @@ int build_pcg(hf_case *C, const std::vector<int32_t> &mptr, const std::vector<in
     struct InstHier {
         std::vector<hf::HostLevel> H;
         std::vector<double> inv;   // row-major
+        solve::HostSolve F;
         std::string err;
     };
     std::vector<InstHier> IH(ni);
@@ -1925,6 +2129,7 @@ int build_pcg(hf_case *C, const std::vector<int32_t> &mptr, const std::vector<in
                 std::vector<double> inv;
                 if (!hf::dense_inverse(last.A, inv)) { ih.err = "singular coarsest AMG level"; continue; }
                 ih.inv = std::move(inv);
+                if (C->use_cg && !C->sie && n <= kSolveMaxRows) ih.F = solve::build(ih.H, C->P.ncell);
             }
         };
         const unsigned nt = std::max(1u, std::min(std::thread::hardware_concurrency(), 32u));
@@ -1937,6 +2142,16 @@ int build_pcg(hf_case *C, const std::vector<int32_t> &mptr, const std::vector<in
             clev[i] = (int)IH[i].H.size() - 1;
         }
     }
+    // the one-launch solve, when every instance's operators fit its encoding
+    // and no instance is beyond the size one cluster is the better choice for.
+    // Not with semi-implicit velocities: their BiCGStab solves turn a last-bit
+    // change of the pressure into a change of the size of their own tolerance
+    // (measured on a 96 x 96 case at rtol 1e-10: 2e-10 of u and 5e-9 of p after
+    // one step), so that form keeps the arithmetic of the level-synchronous
+    // kernels.
+    bool fused = C->use_cg && amg && !C->sie;
+    for (int i = 0; i < ni && fused; i++) fused = IH[i].F.ok;
+    C->fused = fused;
     int nlev = 1;
     for (int i = 0; i < ni; i++) nlev = std::max(nlev, clev[i] + 1);
     C->nlev = nlev;
@@ -1967,6 +2182,17 @@ int build_pcg(hf_case *C, const std::vector<int32_t> &mptr, const std::vector<in
         LevelHost &h = LH[l];
         h.n = off[l][ni];
         C->lrows[l] = h.n;
+        if (fused) {
+            if (l == 0) h.ablk = block_table(off, tail, 0, false);
+            for (int i = 0; i < ni; i++) {
+                if (clev[i] < l) continue;
+                const hf::HostLevel &hl = IH[i].H[l];
+                C->lnnz_a[l] += (int64_t)hl.A.col.size();
+                C->lnnz_p[l] += (int64_t)hl.P.col.size();
+                C->lnnz_r[l] += (int64_t)hl.R.col.size();
+            }
+            continue;
+        }
         if (l == 0) {
             C->lnnz_a[0] = (int64_t)mcol.size();
             if (amg) {
@@ -2053,7 +2279,7 @@ int build_pcg(hf_case *C, const std::vector<int32_t> &mptr, const std::vector<in
     }
 
     // every index the kernels follow must stay inside its array
-    for (int l = 0; l < nlev; l++) {
+    for (int l = 0; l < (fused ? 1 : nlev); l++) {
         const LevelHost &h = LH[l];
         const int nn = l + 1 < nlev ? LH[l + 1].n : 0;
         auto cols_ok = [](const std::vector<int32_t> &p, const std::vector<int32_t> &c, size_t rows, int ncol) {
@@ -2063,7 +2289,7 @@ int build_pcg(hf_case *C, const std::vector<int32_t> &mptr, const std::vector<in
             return true;
         };
         bool ok = l == 0 || cols_ok(h.Ap, h.Ac, h.n, h.n);
-        if (ok && l + 1 < nlev) ok = cols_ok(h.Pp, h.Pc, h.n, nn) && cols_ok(h.Rp, h.Rc, nn, h.n);
+        if (ok && l + 1 < nlev && !fused) ok = cols_ok(h.Pp, h.Pc, h.n, nn) && cols_ok(h.Rp, h.Rc, nn, h.n);
         for (const std::vector<Blk> *t : {&h.sblk, &h.ablk})
             for (const Blk &b : *t) {
                 if (b.row0 < 0 || b.cnt <= 0 || b.cnt > kBlockRows || b.row0 + b.cnt > h.n) ok = false;
@@ -2114,7 +2340,7 @@ int build_pcg(hf_case *C, const std::vector<int32_t> &mptr, const std::vector<in
     }
     // template forms of the operators and transfers the level-synchronous
     // kernels read (levels above the last tail start); the tails keep CSR
-    if (amg) {
+    if (amg && !fused) {
         std::vector<std::thread> th;
         for (int l = 0; l < C->nreg && l + 1 < nlev; l++) {
             LevelHost &h = LH[l];
@@ -2130,11 +2356,11 @@ int build_pcg(hf_case *C, const std::vector<int32_t> &mptr, const std::vector<in
     Arena ar;
     ar.add(nullptr, 8);   // offset 0 stays unused: a zero offset means "absent"
     std::vector<LevelOff> LO(nlev);
-    if (amg)
+    if (amg && !fused)
         for (int l = 0; l < nlev; l++)
             LO[l] = mixed ? place_level<float>(ar, LH[l], l == 0) : place_level<double>(ar, LH[l], l == 0);
     std::vector<size_t> inv_off(ni, 0);
-    if (amg)
+    if (amg && !fused)
         for (int i = 0; i < ni; i++)
             inv_off[i] = mixed ? ar.vec(cast_vec<float>(IH[i].inv)) : ar.vec(IH[i].inv);
     const int n = C->P.ncell;
@@ -2217,7 +2443,20 @@ int build_pcg(hf_case *C, const std::vector<int32_t> &mptr, const std::vector<in
         C->pa32 = (float *)(base + o_pa32);
         C->pb32 = (float *)(base + o_pb32);
     }
-    if (amg) {
+    if (fused) {
+        int rc = HF_OK;
+        std::vector<const solve::HostSolve *> F(ni);
+        std::vector<const std::vector<double> *> inv(ni);
+        for (int i = 0; i < ni; i++) {
+            F[i] = &IH[i].F;
+            inv[i] = &IH[i].inv;
+            C->coarse_rows += F[i]->nc;
+            C->coarse_dense += (int64_t)F[i]->nc * F[i]->nc;
+        }
+        rc = mixed ? build_solve<float>(C, F, inv, C->si32) : build_solve<double>(C, F, inv, C->si64);
+        if (rc) return rc;
+    }
+    if (amg && !fused) {
         for (int l = 0; l < nlev; l++) {
             if (mixed) {
                 const TRows<float> At32{G.A.rd, G.A.toff, (const float *)(base + o_tval32)};
@@ -2347,6 +2586,43 @@ void enqueue_body(hf_case *C, cudaStream_t st, cudaGraphConditionalHandle cond, 
         launch_pdl(k_pcg_update, C->G.nblk, kBlock, st, C->G, (const double *)pn, cond, set);
         kernels += 2;
     }
+}
+
+// The whole solve as one launch per cluster size, side by side on streams
+// forked from st and joined to it (under capture: parallel branches)
+int enqueue_solve(hf_case *C, cudaStream_t st, int &kernels)
+{
+    auto launch = [&](const hf_case::SolveLaunch &L, cudaStream_t on) -> cudaError_t {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)(L.count * L.cluster));
+        cfg.blockDim = dim3((unsigned)L.threads);
+        cfg.dynamicSmemBytes = L.smem;
+        cfg.stream = on;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = (unsigned)L.cluster;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        kernels++;
+        const PcgFine &G = C->G;
+        if (C->mixed)
+            return cudaLaunchKernelEx(&cfg, solve_kernel<float>(L.fine), G,
+                                      SolveArgs<float>{C->si32, G.r32, G.z32, C->pa32, G.q32, G.e32, L.first});
+        return cudaLaunchKernelEx(&cfg, solve_kernel<double>(L.fine), G,
+                                  SolveArgs<double>{C->si64, G.r, G.z, C->pa, G.q, nullptr, L.first});
+    };
+    if (C->solves.size() > 1) HF_CK(cudaEventRecord(C->solve_events[0], st));
+    for (size_t k = 0; k < C->solves.size(); k++) {
+        cudaStream_t on = k ? C->solve_streams[k - 1] : st;
+        if (k) HF_CK(cudaStreamWaitEvent(on, C->solve_events[0], 0));
+        HF_CK(launch(C->solves[k], on));
+    }
+    for (size_t k = 1; k < C->solves.size(); k++) {
+        HF_CK(cudaEventRecord(C->solve_events[k], C->solve_streams[k - 1]));
+        HF_CK(cudaStreamWaitEvent(st, C->solve_events[k], 0));
+    }
+    return HF_OK;
 }
 
 // One semi-implicit velocity system: BiCGStab with Jacobi scaling on Mu from
@@ -2623,7 +2899,11 @@ int eager_step(hf_case *C)
     if (C->sie_rc) return C->sie_rc;
     // the mixed form: up to kMaxSweeps inner solves, each followed by the FP64
     // correction; the plain form: one solve
-    const int sweeps = C->mixed ? kMaxSweeps : 1;
+    const int sweeps = C->fused ? 0 : C->mixed ? kMaxSweeps : 1;
+    if (C->fused) {
+        int rc = enqueue_solve(C, C->stream, fixed);
+        if (rc) return rc;
+    }
     for (int sw = 0; sw < sweeps; sw++) {
         for (;;) {
             body = 0;
@@ -2661,8 +2941,9 @@ int capture_step(hf_case *C, DevFields F, cudaGraph_t *gout)
     // the iterations: a conditional WHILE node after everything captured so far;
     // the mixed form has kMaxSweeps of them, each followed by its FP64
     // correction, which sets the next one's condition
-    const int sweeps = C->mixed ? kMaxSweeps : 1;
-    cudaError_t e = cudaSuccess;
+    const int sweeps = C->fused ? 0 : C->mixed ? kMaxSweeps : 1;
+    const int solve_rc = C->fused ? enqueue_solve(C, st, fixed) : HF_OK;
+    cudaError_t e = solve_rc ? cudaErrorUnknown : cudaSuccess;
     cudaGraphConditionalHandle cond[kMaxSweeps] = {};
     bool have[kMaxSweeps] = {};
     cudaGraph_t g = nullptr;
@@ -2797,7 +3078,8 @@ int collect_phases(hf_case *C)
     C->phase_launches[HF_PHASE_VELOCITY] += 1 + (C->P.vr.n ? 1 : 0) + (rk ? 1 : 0);
     if (C->P.vr.n) C->phase_launches[HF_PHASE_VELOCITY_ROWS] += 1;
     C->phase_launches[HF_PHASE_POISSON_INIT] += 2;
-    C->phase_launches[HF_PHASE_POISSON_ITER] += (C->h_ctl->total_bodies - C->bodies0) * C->body_kernels;
+    C->phase_launches[HF_PHASE_POISSON_ITER] += C->fused ? (int64_t)C->solves.size()
+                                                         : (C->h_ctl->total_bodies - C->bodies0) * C->body_kernels;
     C->phase_launches[HF_PHASE_FINAL] += 2;
     return HF_OK;
 }
@@ -3917,6 +4199,8 @@ extern "C" void hf_case_destroy(hf_case *C)
     delete C->h_scal;
     delete[] C->h_S;
     delete C->h_ctl;
+    for (cudaStream_t q : C->solve_streams) cudaStreamDestroy(q);
+    for (cudaEvent_t q : C->solve_events) cudaEventDestroy(q);
     if (C->body_stream) cudaStreamDestroy(C->body_stream);
     if (C->stream) cudaStreamDestroy(C->stream);
     delete C;
