@@ -1906,169 +1906,58 @@ constexpr int kSolveMaxRows = 1 << 19;
 // The one-launch solves' tables of every instance on the device, the instances
 // grouped by cluster size (one launch each), largest first.
 template <typename T>
-auto solve_kernel(int fine) -> void (*)(PcgFine, SolveArgs<T>)
+auto solve_kernel(int fine) -> void (*)(PcgFine, SolveArgs<T>, int)
 {
     constexpr bool mix = std::is_same<T, float>::value;
     return fine == 5 ? k_solve<T, mix, 5> : fine == 7 ? k_solve<T, mix, 7> : k_solve<T, mix, 0>;
 }
 
 template <typename T>
-int build_solve(hf_case *C, const std::vector<const solve::HostSolve *> &F, const std::vector<const std::vector<double> *> &inv,
-                SInst<T> *&dev)
+int build_solve(hf_case *C, std::vector<solve::Packed<T>> &K, const std::vector<const solve::HostSolve *> &F, SInst<T> *&dev)
 {
     const int ni = C->ninst;
     std::vector<int> order(ni);
     for (int i = 0; i < ni; i++) order[i] = i;
     auto rows = [&](int i) { return C->coff[i + 1] - C->coff[i]; };
-    auto key = [&](int i) { return F[i]->cluster * 64 + F[i]->fine; };
+    auto key = [&](int i) {
+        return ((long)F[i]->cluster * 256 + F[i]->fine) * 64 + F[i]->threads / 32;
+    };
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
         if (key(a) != key(b)) return key(a) > key(b);
         return rows(a) > rows(b);
     });
     Arena ar;
-    std::vector<SInst<T>> I(ni);
     struct Where {
-        size_t tables, rows_r, rows_u, gvec, rng;
+        size_t tables, rank_tables, ranks, rng;
     };
     std::vector<Where> W(ni);
-    std::vector<size_t> smem(ni, 0);
-    for (int k = 0; k < ni; k++) {
-        const int i = order[k];
-        const solve::HostSolve &f = *F[i];
-        const int C0 = f.cluster;
-        SInst<T> &o = I[k];
-        memset(&o, 0, sizeof o);
-        o.inst = i;
-        o.row0 = C->coff[i];
-        o.n = rows(i);
-        o.s = f.s;
-        o.clev = f.clev;
-        o.nc = f.nc;
-        // shared memory, in this order as far as each piece fits: the tail's
-        // vectors (always), the vectors with halos, the finest vectors' own
-        // rows, row descriptors and operator tables of the finest level, the
-        // tail's, and the levels' between
-        size_t at = 0;
-        auto take = [&](size_t bytes, size_t keep = 0) -> uint32_t {
-            bytes = (bytes + 15) & ~size_t(15);
-            if (at + bytes + keep > kSolveSmem) return kSolveGlobal;
-            const uint32_t r = (uint32_t)at;
-            at += bytes;
-            return r;
-        };
-        auto elems = [&](uint32_t b) { return b == kSolveGlobal ? b : (uint32_t)(b / sizeof(T)); };
-        const int nl = (int)f.L.size();
-        for (int l = std::max(1, f.s); l < f.clev; l++) {
-            o.L[l].vb = elems(take(sizeof(T) * f.L[l].n));
-            o.L[l].vo = elems(take(sizeof(T) * f.L[l].n));
-        }
-        o.cvec = elems(take(sizeof(T) * 2 * f.nc));
-        o.vr = take(sizeof(T) * f.held[0]);
-        o.vz = take(sizeof(T) * f.held[1]);
-        size_t g = 0;
-        for (int l = 1; l < f.s; l++) {
-            o.L[l].vb = elems(take(sizeof(T) * f.held[2 * l]));
-            o.L[l].vo = elems(take(sizeof(T) * f.held[2 * l + 1]));
-            o.L[l].gb = (uint32_t)g;
-            o.L[l].go = (uint32_t)(g + f.L[l].n);
-            g += 2 * (size_t)f.L[l].n;
-        }
-        const size_t own = (o.n + C0 - 1) / C0, reserve = 48 * 1024;
-        o.vq = take(sizeof(T) * own, reserve);
-        o.vp = take(sizeof(T) * own, reserve);
-        o.vx = take((C->mixed ? sizeof(T) : sizeof(double)) * own, reserve);
-        std::vector<uint2> rr;
-        std::vector<uint4> ru;
-        std::vector<char> blob;
-        for (int l = 0; l < nl; l++) {
-            const solve::HostSolve::Level &h = f.L[l];
-            SLevel &v = o.L[l];
-            v.n = h.n;
-            v.lanes_r = h.lanes_r;
-            v.lanes_u = h.lanes_u;
-            v.row_r = (uint32_t)rr.size();
-            v.row_u = (uint32_t)ru.size();
-            rr.insert(rr.end(), h.rows_r.begin(), h.rows_r.end());
-            ru.insert(ru.end(), h.rows_u.begin(), h.rows_u.end());
-        }
-        auto part = [&](const void *data, size_t bytes, size_t keep = 0) {
-            STab t;
-            t.g = (uint32_t)blob.size();
-            t.bytes = (uint32_t)((bytes + 15) & ~size_t(15));
-            t.s = take(bytes, keep);
-            blob.insert(blob.end(), (const char *)data, (const char *)data + bytes);
-            blob.resize((blob.size() + 15) & ~size_t(15), 0);
-            return t;
-        };
-        auto ents = [&](const std::vector<int32_t> &off, const std::vector<double> &val) {
-            std::vector<SEnt<T>> e(off.size());
-            memset(e.data(), 0, e.size() * sizeof(SEnt<T>));
-            for (size_t q = 0; q < e.size(); q++) {
-                e[q].off = off[q];
-                e[q].v = (T)val[q];
-            }
-            return part(e.data(), e.size() * sizeof(SEnt<T>));
-        };
-        auto level_rows = [&](int l) {
-            // own rows of a distributed level, all of a tail level's
-            const size_t nu = f.L[l].n, nr = f.L[l].rows_r.size(), d = l < f.s ? C0 : 1;
-            o.L[l].srow_u = take(sizeof(uint4) * ((nu + d - 1) / d));
-            o.L[l].srow_r = take(sizeof(uint2) * ((nr + d - 1) / d));
-        };
-        auto level_tabs = [&](int l) {
-            o.L[l].m = ents(f.L[l].off_m, f.L[l].v_m);
-            o.L[l].p = ents(f.L[l].off_p, f.L[l].v_p);
-            o.L[l].r = ents(f.L[l].off_r, f.L[l].v_r);
-        };
-        o.a = ents(f.L[0].off_m, f.L[0].v_a);
-        level_tabs(0);
-        level_rows(0);
-        {
-            std::vector<T> d(inv[i]->begin(), inv[i]->end());
-            o.inv = part(d.data(), d.size() * sizeof(T));
-        }
-        for (int l = f.clev - 1; l >= std::max(1, f.s); l--) {
-            level_rows(l);
-            level_tabs(l);
-        }
-        for (int l = f.s - 1; l > 0; l--) {
-            level_rows(l);
-            level_tabs(l);
-        }
-        if (C->mixed) {
-            std::vector<SEnt<double>> e(f.L[0].off_m.size());
-            for (size_t q = 0; q < e.size(); q++) e[q] = SEnt<double>{f.L[0].v_a[q], f.L[0].off_m[q], 0};
-            o.a64 = part(e.data(), e.size() * sizeof(SEnt<double>));
-        }
-        smem[k] = at;
-        W[k] = Where{ar.vec(blob), ar.vec(rr), ar.vec(ru), ar.zeros<T>(g), ar.vec(f.rng)};
-    }
+    for (int i = 0; i < ni; i++)
+        W[i] = Where{ar.vec(K[i].tables), ar.vec(K[i].rank_tables), ar.vec(K[i].ranks), ar.vec(F[i]->rng)};
     char *base = nullptr;
     HF_CK(cudaMallocAsync((void **)&base, ar.host.size(), C->stream));
     C->owned.push_back(base);
     C->bytes += (double)ar.host.size();
     HF_CK(cudaMemcpyAsync(base, ar.host.data(), ar.host.size(), cudaMemcpyHostToDevice, C->stream));
+    std::vector<SInst<T>> I(ni);
     for (int k = 0; k < ni; k++) {
-        I[k].tables = base + W[k].tables;
-        I[k].rows_r = (const uint2 *)(base + W[k].rows_r);
-        I[k].rows_u = (const uint4 *)(base + W[k].rows_u);
-        I[k].gvec = (T *)(base + W[k].gvec);
-        I[k].rng = (const int4 *)(base + W[k].rng);
+        const int i = order[k];
+        I[k] = K[i].inst;
+        I[k].inst = i;
+        I[k].row0 = C->coff[i];
+        I[k].tables = base + W[i].tables;
+        I[k].rank_tables = base + W[i].rank_tables;
+        I[k].ranks = (const SRank *)(base + W[i].ranks);
+        I[k].rng = (const int4 *)(base + W[i].rng);
     }
     int rc = upload(C->owned, &dev, I.data(), I.size(), C->bytes, C->stream);
     if (rc) return rc;
     HF_CK(cudaStreamSynchronize(C->stream));   // the host copies go away with this function
     for (int k = 0; k < ni;) {
         const solve::HostSolve &f = *F[order[k]];
-        int e = k, own = 0;
+        int e = k;
         size_t most = 0;
-        for (; e < ni && key(order[e]) == key(order[k]); e++) {
-            most = std::max(most, smem[e]);
-            own = std::max(own, (I[e].n + f.cluster - 1) / f.cluster);
-        }
-        // one row per thread as far as a block goes
-        int threads = std::min(kSolveThreads, std::max(256, (own + 31) / 32 * 32));
-        C->solves.push_back(hf_case::SolveLaunch{k, e - k, f.cluster, f.fine, threads, most});
+        for (; e < ni && key(order[e]) == key(order[k]); e++) most = std::max(most, K[order[e]].smem);
+        C->solves.push_back(hf_case::SolveLaunch{k, e - k, f.cluster, f.fine, f.threads, most});
         auto *kern = solve_kernel<T>(f.fine);
         HF_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSolveSmem));
         HF_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
@@ -2151,6 +2040,27 @@ int build_pcg(hf_case *C, const std::vector<int32_t> &mptr, const std::vector<in
     // kernels.
     bool fused = C->use_cg && amg && !C->sie;
     for (int i = 0; i < ni && fused; i++) fused = IH[i].F.ok;
+    std::vector<solve::Packed<double>> K64;
+    std::vector<solve::Packed<float>> K32;
+    if (fused) {
+        if (mixed) K32.resize(ni);
+        else K64.resize(ni);
+        std::atomic<int> next{0};
+        std::atomic<bool> all{true};
+        auto work = [&]() {
+            for (int i; (i = next++) < ni;) {
+                if (mixed) K32[i] = solve::pack<float>(IH[i].F, IH[i].inv, true);
+                else K64[i] = solve::pack<double>(IH[i].F, IH[i].inv, false);
+                if (!(mixed ? K32[i].ok : K64[i].ok)) all = false;
+            }
+        };
+        const unsigned nt = std::max(1u, std::min(std::thread::hardware_concurrency(), 32u));
+        std::vector<std::thread> th;
+        for (unsigned t = 0; t + 1 < nt && (int)t + 1 < ni; t++) th.emplace_back(work);
+        work();
+        for (auto &t : th) t.join();
+        fused = all;
+    }
     C->fused = fused;
     int nlev = 1;
     for (int i = 0; i < ni; i++) nlev = std::max(nlev, clev[i] + 1);
@@ -2444,16 +2354,13 @@ int build_pcg(hf_case *C, const std::vector<int32_t> &mptr, const std::vector<in
         C->pb32 = (float *)(base + o_pb32);
     }
     if (fused) {
-        int rc = HF_OK;
         std::vector<const solve::HostSolve *> F(ni);
-        std::vector<const std::vector<double> *> inv(ni);
         for (int i = 0; i < ni; i++) {
             F[i] = &IH[i].F;
-            inv[i] = &IH[i].inv;
             C->coarse_rows += F[i]->nc;
             C->coarse_dense += (int64_t)F[i]->nc * F[i]->nc;
         }
-        rc = mixed ? build_solve<float>(C, F, inv, C->si32) : build_solve<double>(C, F, inv, C->si64);
+        const int rc = mixed ? build_solve<float>(C, K32, F, C->si32) : build_solve<double>(C, K64, F, C->si64);
         if (rc) return rc;
     }
     if (amg && !fused) {
@@ -2608,9 +2515,9 @@ int enqueue_solve(hf_case *C, cudaStream_t st, int &kernels)
         const PcgFine &G = C->G;
         if (C->mixed)
             return cudaLaunchKernelEx(&cfg, solve_kernel<float>(L.fine), G,
-                                      SolveArgs<float>{C->si32, G.r32, G.z32, C->pa32, G.q32, G.e32, L.first});
+                                      SolveArgs<float>{C->si32, G.r32, C->pa32, G.e32, L.first}, L.fine);
         return cudaLaunchKernelEx(&cfg, solve_kernel<double>(L.fine), G,
-                                  SolveArgs<double>{C->si64, G.r, G.z, C->pa, G.q, nullptr, L.first});
+                                  SolveArgs<double>{C->si64, G.r, C->pa, nullptr, L.first}, L.fine);
     };
     if (C->solves.size() > 1) HF_CK(cudaEventRecord(C->solve_events[0], st));
     for (size_t k = 0; k < C->solves.size(); k++) {

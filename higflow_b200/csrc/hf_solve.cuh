@@ -5,40 +5,45 @@
 // What bounds it: at the sizes of single cases and of the batches' instances
 // (10^3 to 10^5 rows) a CG iteration of level-synchronous launches is a chain of
 // 8 to 20 dependent kernels of 4 to 5 us each.  Here the phases are separated by
-// the hardware's cluster barrier instead, and there are fewer of them:
+// the hardware's cluster barrier instead (400 to 600 cycles), and there are few
+// of them, two per level and three for the finest:
 //  - the V-cycle's smoothing is folded into its transfers when the case is
 //    created, so each level takes one phase down and one up:
 //      b_{l+1} = Rt b_l,  Rt = R (I - A w D^-1)   (pre-smoothing, residual, R)
 //      out_l = Mt b_l + Pt out_{l+1},  Mt = 2 w D^-1 - w D^-1 A w D^-1,
 //      Pt = (I - w D^-1 A) P                      (prolongation, post-smoothing)
-//    (the same V-cycle in exact arithmetic);
-//  - the small levels (kSolveTail rows and below) run in every CTA of the
-//    cluster for itself, so they need block barriers only;
-//  - q = A p is carried as q = A z + beta q, so p has no neighbour reads;
+//    (the same V-cycle in exact arithmetic); the dense coarsest solve runs in
+//    every CTA for itself;
+//  - q = A p is carried as q = A z + beta q, so p has no neighbour reads, and r
+//    is updated over a CTA's halo as well as its own rows from the halo of q, so
+//    the update and the first phase down need no barrier between them;
 //  - each dot product's partial sums travel with the barrier that follows it.
-// And a phase is short: a CTA owns a contiguous range of every level's rows and
-// holds the vectors over that range and the columns its rows reach (its halo)
-// in shared memory.  The owner of a value stores it to its own copy and to the
-// halo copies of the CTAs that read it (distributed shared memory), so every
-// gather is a local shared-memory load.  The operators are row templates (a few
-// hundred entries per level on a uniform grid) in shared memory too.  What does
-// not fit stays in global memory (L2) behind the same indexing.
+// A phase is short because nothing in it leaves the SM: a CTA owns a contiguous
+// range of every level's rows and holds the vectors over that range and the
+// columns its rows reach (its halo) in shared memory.  The owner of a value
+// stores it to its own copy and to the halo copies of the CTAs that read it
+// (distributed shared memory), so every gather is a local shared-memory load.
+// The operators lie in shared memory too, as far as they fit: the finest level's
+// as row templates (a few hundred entries on a uniform grid, read by most of a
+// warp at once), the coarse levels' as the CTA's own rows in slices of 32
+// threads (rows there rarely share a template: 32 threads reading 32 templates
+// conflict on the banks), with columns as 16-bit shared-memory element indices.
 //
 // Partial sums are added in a fixed order: the same results on every run.
 #pragma once
 
 #include <cstdint>
 
-constexpr int kSolveThreads = 1024;
+constexpr int kSolveThreads = 1024;          // most threads of a CTA
 constexpr int kSolveWarps = kSolveThreads / 32;
-constexpr int kSolveTail = 1024;             // largest level run by every CTA for itself
-constexpr int kSolveSmem = 206 * 1024;       // dynamic shared memory
-constexpr int kSolveLenBits = 10;            // rows of up to 1023 entries, 2^22 entries per operator
+constexpr int kSolveSmem = 208 * 1024;       // dynamic shared memory
+constexpr int kSolveLenBits = 10;            // template rows of up to 1023 entries, 2^22 entries per operator
 constexpr int kSolveMaxCluster = 16;
-constexpr int kSolveVecs = 2 * kMaxLevels;   // vectors with halos: r, z, then b and out of the levels between
+constexpr int kSolveVecs = 2 * kMaxLevels;   // vectors with halos: r (and q), z, then b and out of the levels between
 constexpr uint32_t kSolveGlobal = 0xffffffffu;   // "not in shared memory"
 
-// one operator entry: column offset from the row's anchor, value
+// one entry of the finest operator's rows: column offset from the row (SInst::a
+// and m: in bytes of T, a64: in rows), value
 template <typename T>
 struct SEnt;
 template <>
@@ -52,95 +57,133 @@ struct __align__(16) SEnt<double> {
     int32_t off, pad;
 };
 
-// an array of the instance's tables: its place in global memory and, when it
-// is copied to shared memory, there (byte offsets)
+// an array of the instance's (or rank's) tables: byte offset in global memory
+// and, when it is copied to shared memory, there
 struct STab {
     uint32_t g, s, bytes;
 };
 
-// one level of one instance (every level but the coarsest).  Row descriptors
-// are (first entry << kSolveLenBits) | entry count.
-struct SLevel {
-    int32_t n;                // rows
-    int32_t lanes_r, lanes_u; // threads per row of the way down (a row of the next level) / up
-    // row descriptors down (uint2: row, anchor) and up (uint4: Mt row, Pt row,
-    // Pt anchor): global arrays; of the levels above the tail every CTA copies
-    // its own rows to shared memory, of the tail all rows
-    uint32_t row_r, row_u;    // first descriptor in SInst::rows_r / rows_u
-    uint32_t srow_r, srow_u;  // their place in shared memory (bytes) or kSolveGlobal
-    STab r, m, p;             // operator tables
-    uint32_t vb, vo;          // vectors b and out: T elements into shared memory (kSolveGlobal: into gvec)
-    uint32_t gb, go;          // ... into SInst::gvec (levels above the tail)
+// An operator's rows of one rank as slices: slice k holds 32 >> lg rows, 1 << lg
+// threads each; the entries of its 32 threads lie side by side, turn by turn
+// (turns ptr[k] to ptr[k + 1]).  t: ptr (padded to 16 bytes), the values, the
+// columns (16-bit element indices into shared memory).
+struct SOp {
+    STab t;
+    int32_t row0, rows, lg, nsl;
+    uint32_t val, idx;        // byte offsets of the values and columns in t
+};
+
+// what one rank of an instance's cluster reads
+struct SRank {
+    SOp down[kMaxLevels];     // Rt of level l (rows: the next level's)
+    SOp up[kMaxLevels];       // Mt and Pt of level l > 0 together; the finest level: Pt
+    STab desc0;               // finest level's own rows: uint2 {Pt template row, Pt anchor (element index) << 16 | Mt/A template}
+    STab desc_r;              // template form of the first way down: uint2 {Rt template row, anchor (element index)}
 };
 
 template <typename T>
 struct SInst {
-    int32_t inst, row0, n, s, clev, nc;      // s: first tail level; nc: rows of the coarsest
-    uint32_t vr, vz, vp, vq, vx;             // finest vectors in shared memory (bytes; vx: x, or e in the mixed form)
-    uint32_t cvec;                           // the coarsest level's vectors (T elements into shared memory)
-    STab a, a64, inv;                        // finest operator (T, FP64), dense inverse
+    int32_t inst, row0, n, clev, nc;         // clev: the coarsest level; nc: its rows
+    int32_t tpl_p, tpl_r, lg_r;              // the finest Pt / Rt as templates; threads per Rt row (log2)
+    uint32_t vr, vq, vz, vp, vx;             // finest vectors in shared memory (bytes; vx: x, or e in the mixed form)
+    uint32_t vb[kMaxLevels], vo[kMaxLevels]; // vectors of the levels between (bytes)
+    uint32_t cvec;                           // the coarsest level's vectors (bytes)
+    STab a, m, a64, inv;                     // finest operator (T), Mt, finest operator (FP64), dense inverse
+    STab tpv, tpo, trv, tro;                 // template entries of Pt / Rt: values, 16-bit column offsets
+    int32_t lvl[kMaxLevels];                 // rows of the levels
     const char *tables;
-    const uint2 *rows_r;
-    const uint4 *rows_u;
-    T *gvec;
+    const char *rank_tables;                 // the ranks' tables (SRank offsets are into these)
+    const SRank *ranks;
     // [kSolveVecs][cluster]: rows [x, y) each rank holds of a vector, and the
     // ranks [z, w] that hold some of its own rows
     const int4 *rng;
-    SLevel L[kMaxLevels];
 };
 
 template <typename T>
 struct SolveArgs {
     const SInst<T> *I;
-    T *r, *z, *p, *q, *e;                    // finest vectors in global memory (e: mixed form only)
+    const T *r;                              // the first residual
+    T *p, *e;                                // where p and e do not fit (e: mixed form only)
     int first;                               // first instance of this launch in I
 };
 
 namespace solve {
 
-namespace cg = ::cooperative_groups;
-
 __device__ __forceinline__ float fma_(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ double fma_(double a, double b, double c) { return __fma_rn(a, b, c); }
 
-// a row's entries k0, k0 + step, ... (two per turn: the host pads rows to an
-// even number of turns) times f
+// Shared memory is addressed by 32-bit byte offsets into the kernel's dynamic
+// part (dyn): the loads are then plain shared-memory loads with 32-bit address
+// arithmetic, where pointers kept in a struct would be generic 64-bit ones (the
+// phases are chains of a few hundred instructions a warp, so these count).
+extern __shared__ __align__(16) char dyn[];
 template <typename T>
-__device__ __forceinline__ T row_part(const SEnt<T> *tab, uint32_t d, int lane, int lanes, const T *f)
+__device__ __forceinline__ T &at(uint32_t off)
 {
-    const SEnt<T> *t = tab + (d >> kSolveLenBits) + lane;
+    return *reinterpret_cast<T *>(dyn + off);
+}
+
+// the address of a shared variable in another CTA of the cluster, and a store to it
+__device__ __forceinline__ uint32_t peer(uint32_t local, int rank)
+{
+    uint32_t a;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(local), "r"(rank));
+    return a;
+}
+__device__ __forceinline__ uint32_t address(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void store_peer(uint32_t a, double v)
+{
+    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
+}
+__device__ __forceinline__ void store_peer(uint32_t a, float v)
+{
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
+}
+
+// a template row's entries lane, lane + lanes, ... (two per turn: the host pads
+// rows to a whole number of turns) times f; val, off: byte offsets of the tables
+template <typename T>
+__device__ __forceinline__ T row_part(uint32_t val, uint32_t off, uint32_t d, int lane, int lanes, uint32_t f)
+{
+    const uint32_t k0 = (d >> kSolveLenBits) + lane;
+    val += k0 * (uint32_t)sizeof(T);
+    off += k0 * 2u;
     int len = (int)(d & ((1u << kSolveLenBits) - 1));
     T s = T(0), u = T(0);
 #pragma unroll 2
     for (; len > 0; len -= 2 * lanes) {
-        const SEnt<T> e0 = t[0], e1 = t[lanes];
-        t += 2 * lanes;
-        s = fma_(e0.v, f[e0.off], s);
-        u = fma_(e1.v, f[e1.off], u);
+        const int o0 = at<int16_t>(off), o1 = at<int16_t>(off + 2u * lanes);
+        s = fma_(at<T>(val), at<T>(f + o0 * (int)sizeof(T)), s);
+        u = fma_(at<T>(val + (uint32_t)sizeof(T) * lanes), at<T>(f + o1 * (int)sizeof(T)), u);
+        val += 2u * (uint32_t)sizeof(T) * lanes;
+        off += 4u * lanes;
     }
     return s + u;
 }
 
-// a row of exactly K entries (shorter rows are padded)
+// a row of exactly K entries (shorter rows are padded); k: entries, K = 0.
+// t: byte offset of the entries, f: of the row's own element
 template <int K, typename T>
-__device__ __forceinline__ T row_fixed(const SEnt<T> *tab, uint32_t d, const T *f)
+__device__ __forceinline__ T row_fixed(uint32_t t, int k, uint32_t f)
 {
-    const SEnt<T> *t = tab + (d >> kSolveLenBits);
     T s = T(0), u = T(0);
+    if (K > 0) {
+        SEnt<T> e[K > 0 ? K : 1];
 #pragma unroll
-    for (int k = 0; k < K; k++) {
-        const SEnt<T> e = t[k];
-        T &a = k & 1 ? u : s;
-        a = fma_(e.v, f[e.off], a);
+        for (int j = 0; j < K; j++) e[j] = at<SEnt<T>>(t + j * (uint32_t)sizeof(SEnt<T>));
+#pragma unroll
+        for (int j = 0; j < K; j++) {
+            T &a = j & 1 ? u : s;
+            a = fma_(e[j].v, at<T>(f + e[j].off), a);
+        }
+    } else {
+#pragma unroll 4
+        for (int j = 0; j < k; j++) {
+            const SEnt<T> e = at<SEnt<T>>(t + j * (uint32_t)sizeof(SEnt<T>));
+            s = fma_(e.v, at<T>(f + e.off), s);
+        }
     }
     return s + u;
-}
-
-// a row of the finest operator: K entries, or any even number (K = 0)
-template <int K, typename T>
-__device__ __forceinline__ T fine_row(const SEnt<T> *tab, uint32_t d, const T *f)
-{
-    return K > 0 ? row_fixed<K>(tab, d, f) : row_part(tab, d, 0, 1, f);
 }
 
 template <typename T>
@@ -151,38 +194,51 @@ __device__ __forceinline__ T lanes_sum(T s, int lanes)
 }
 
 struct Team {
-    int rank, size;
-    double (*slot)[kSolveMaxCluster][kSolveWarps];   // [2][rank][warp] partial sums, double buffered
-    int par;
+    int rank, size, par;
+    double (*slot)[kSolveMaxCluster];   // [2][rank] partial sums, double buffered
+    double *warp;                       // per-warp partial sums (zero beyond the block's warps)
 };
 
+// every thread of the cluster; what was written before is visible after
 __device__ __forceinline__ void team_sync(const Team &t)
 {
-    if (t.size > 1) cg::this_cluster().sync();
-    else __syncthreads();
+    if (t.size > 1) {
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    } else {
+        __syncthreads();
+    }
 }
 
-// sum over the cluster, the same value in every thread; a team barrier: what
-// was written before it is visible to every thread of the cluster after it
+// sum over the cluster, the same value in every thread; a team barrier
 __device__ __forceinline__ double team_sum(Team &t, double v)
 {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (lane == 0) t.warp[wid] = v;
+    __syncthreads();
     t.par ^= 1;
-    double *mine = &t.slot[t.par][t.rank][wid];
-    if (t.size > 1) {
-        if (lane < t.size) *cg::this_cluster().map_shared_rank(mine, lane) = v;
-    } else if (lane == 0) {
-        *mine = v;
+    double *mine = &t.slot[t.par][t.rank];
+    if (wid == 0) {
+        v = t.warp[lane];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if (t.size > 1) {
+            if (lane < t.size) store_peer(peer(address(mine), lane), v);
+        } else if (lane == 0) {
+            *mine = v;
+        }
     }
     team_sync(t);
-    // (the slots of warps that do not exist stay zero)
-    double s = 0.0;
-    for (int k = 0; k < t.size; k++) s += t.slot[t.par][k][lane];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    return s;
+    const double2 *s2 = reinterpret_cast<const double2 *>(t.slot[t.par]);
+    double s = 0.0, u = 0.0;
+    for (int k = 0; 2 * k < t.size; k++) {
+        const double2 w = s2[k];
+        s += w.x;
+        u += w.y;   // (zero beyond the cluster)
+    }
+    return s + u;
 }
 
 // rows [lo, hi) of rank k of a level of n rows
@@ -193,96 +249,102 @@ __host__ __device__ __forceinline__ void rank_rows(int k, int size, int n, int &
     hi = lo + ch < n ? lo + ch : n;
 }
 
-// A vector by global row index: at[i] for the rows this CTA holds.  put()
-// stores an own row's value, to the other holders' copies too: rows in
-// [own_lo, own_hi) have none.
+// A vector over the rows this CTA holds: row i at byte offset base + i *
+// sizeof(T).  put() stores an own row's value, to the other holders' copies too:
+// rows in [own_lo, own_hi) have none.
 template <typename T>
 struct Vec {
-    T *at;
-    T *sh;              // this CTA's copy (null: global memory)
+    uint32_t base;
+    uint32_t sh;        // shared address of this CTA's copy
     const int4 *rng;    // per rank
     int rank, klo, khi, own_lo, own_hi;
+    __device__ __forceinline__ uint32_t row(int i) const { return base + (uint32_t)i * (uint32_t)sizeof(T); }
+    __device__ __forceinline__ T get(int i) const { return solve::at<T>(row(i)); }
     __device__ __forceinline__ void put(int i, T v) const
     {
-        at[i] = v;
-        if (i < own_lo || i >= own_hi) put_far(i, v);
-    }
-    __device__ __forceinline__ void put_far(int i, T v) const
-    {
+        solve::at<T>(row(i)) = v;
+        if (i >= own_lo && i < own_hi) return;
         for (int k = klo; k <= khi; k++) {
-            const int4 g = rng[k];
-            if (k != rank && i >= g.x && i < g.y) cg::this_cluster().map_shared_rank(sh, k)[i - g.x] = v;
+            const int2 g = *reinterpret_cast<const int2 *>(rng + k);
+            if (k != rank && i >= g.x && i < g.y) store_peer(peer(sh + (uint32_t)(i - g.x) * (uint32_t)sizeof(T), k), v);
         }
     }
 };
 
-// what a CTA needs of a level, resolved once per solve
-template <typename T>
-struct Plan {
-    const SEnt<T> *tr, *tm, *tp;
-    const uint2 *rr;          // by row
-    const uint4 *ru;
-    Vec<T> b, o;              // by row (the tail's: shared, no halo)
-    int rlo, rhi, ulo, uhi;   // own rows of the way down (the next level's) and up
-    int lr, lu;               // log2 of the threads per row
+// a rank's operator, resolved once per solve: in shared memory (byte offsets) or
+// global (g)
+struct Op {
+    const char *g;
+    uint32_t ptr, val, idx;
+    int row0, rows, lg, nsl;
 };
 
-// the own rows of the operator down to the next level: put(row, value, lane)
-// by every lane of the row
-template <typename T, typename Put>
-__device__ __forceinline__ void down(const Plan<T> &P, const T *b, Put put)
+// this thread's part of slice k
+template <typename T>
+__device__ __forceinline__ T slice_part(const Op &P, int k)
 {
-    const int lr = P.lr, hi = P.rhi, step = blockDim.x >> lr, lane = threadIdx.x & ((1 << lr) - 1);
-    const SEnt<T> *tab = P.tr;
-    const uint2 *rows = P.rr;
-    for (int base = P.rlo; base < hi; base += step) {
-        const int i = base + (threadIdx.x >> lr);
-        const uint2 d = i < hi ? rows[i] : make_uint2(0u, 0u);
-        const T s = lanes_sum(row_part(tab, d.x, lane, 1 << lr, b + (int)d.y), 1 << lr);
-        if (i < hi) put(i, s, lane);
+    const int lane = threadIdx.x & 31;
+    T s = T(0);
+    if (!P.g) {
+        const uint32_t a = at<uint32_t>(P.ptr + 4u * k);
+        int len = (int)(at<uint32_t>(P.ptr + 4u * k + 4u) - a);
+        uint32_t val = P.val + (a * 32u + lane) * (uint32_t)sizeof(T), idx = P.idx + (a * 32u + lane) * 2u;
+#pragma unroll 4
+        for (; len > 0; len--, val += 32u * (uint32_t)sizeof(T), idx += 64u)
+            s = fma_(at<T>(val), at<T>(at<uint16_t>(idx) * (uint32_t)sizeof(T)), s);
+        return s;
     }
+    const uint32_t *ptr = reinterpret_cast<const uint32_t *>(P.g + P.ptr);
+    const uint32_t a = __ldg(ptr + k);
+    int len = (int)(__ldg(ptr + k + 1) - a);
+    const T *val = reinterpret_cast<const T *>(P.g + P.val) + a * 32 + lane;
+    const uint16_t *idx = reinterpret_cast<const uint16_t *>(P.g + P.idx) + a * 32 + lane;
+#pragma unroll 8
+    for (; len > 0; len--, val += 32, idx += 32) s = fma_(__ldg(val), at<T>(__ldg(idx) * (uint32_t)sizeof(T)), s);
+    return s;
 }
 
-// out_l = Mt b_l + Pt e on the own rows
+// every own row of the operator: put(row, value, lane) by every lane of the row
 template <typename T, typename Put>
-__device__ __forceinline__ void up(const Plan<T> &P, const T *b, const T *e, Put put)
+__device__ __forceinline__ void apply(const Op &O, Put put)
 {
-    const int lu = P.lu, hi = P.uhi, step = blockDim.x >> lu, lane = threadIdx.x & ((1 << lu) - 1);
-    const SEnt<T> *tm = P.tm, *tp = P.tp;
-    const uint4 *rows = P.ru;
-    for (int base = P.ulo; base < hi; base += step) {
-        const int i = base + (threadIdx.x >> lu);
-        const uint4 d = i < hi ? rows[i] : make_uint4(0u, 0u, 0u, 0u);
-        T s = row_part(tm, d.x, lane, 1 << lu, b + i);
-        s += row_part(tp, d.y, lane, 1 << lu, e + (int)d.z);
-        s = lanes_sum(s, 1 << lu);
-        if (i < hi && lane == 0) put(i, s);
+    const Op P = O;
+    const int warps = blockDim.x >> 5, lane = threadIdx.x & 31;
+    for (int k = threadIdx.x >> 5; k < P.nsl; k += warps) {
+        const T s = lanes_sum(slice_part<T>(P, k), 1 << P.lg);
+        const int i = (k << (5 - P.lg)) + (lane >> P.lg);
+        if (i < P.rows) put(P.row0 + i, s, lane & ((1 << P.lg) - 1));
     }
 }
 
 }  // namespace solve
 
-// K: entries of the finest operator's rows (5: 2D, 7: 3D uniform grids), 0: any
+// K: entries of the finest operator's rows (5: 2D, 7: 3D uniform grids), 0: see kf
 template <typename T, bool MIX, int K>
-__global__ void __launch_bounds__(kSolveThreads, 1) k_solve(PcgFine G, SolveArgs<T> A)
+__global__ void __launch_bounds__(kSolveThreads, 1) k_solve(PcgFine G, SolveArgs<T> A, int kf)
 {
-    extern __shared__ __align__(16) char dyn[];
+    using solve::at;
     __shared__ SInst<T> I;
-    __shared__ solve::Plan<T> plan[kMaxLevels];
-    __shared__ double slot[2][kSolveMaxCluster][kSolveWarps];
+    __shared__ SRank Rk;
+    __shared__ solve::Op od[kMaxLevels], ou[kMaxLevels];
+    __shared__ solve::Vec<T> vb[kMaxLevels], vo[kMaxLevels];
+    __shared__ __align__(16) double slot[2][kSolveMaxCluster];
+    __shared__ double warp_sums[kSolveWarps];
     __shared__ int4 rng[kSolveVecs][kSolveMaxCluster];
-    namespace cg = ::cooperative_groups;
     const int tid = threadIdx.x, nt = blockDim.x;
+    constexpr uint32_t kT = (uint32_t)sizeof(T), kE = (uint32_t)sizeof(SEnt<T>);
     solve::Team t;
-    t.rank = (int)cg::this_cluster().block_rank();
-    t.size = (int)cg::this_cluster().num_blocks();
+    t.rank = (int)cooperative_groups::this_cluster().block_rank();
+    t.size = (int)cooperative_groups::this_cluster().num_blocks();
     t.slot = slot;
+    t.warp = warp_sums;
     t.par = 0;
-    {
-        const uint32_t *src = reinterpret_cast<const uint32_t *>(A.I + A.first + blockIdx.x / t.size);
-        for (int k = tid; k < (int)(sizeof(SInst<T>) / 4); k += nt) reinterpret_cast<uint32_t *>(&I)[k] = src[k];
-        for (int k = tid; k < 2 * kSolveMaxCluster * kSolveWarps; k += nt) (&slot[0][0][0])[k] = 0.0;
-    }
+    auto copy4 = [&](void *to, const void *from, int bytes) {
+        for (int k = tid; k < bytes / 4; k += nt) static_cast<uint32_t *>(to)[k] = static_cast<const uint32_t *>(from)[k];
+    };
+    copy4(&I, A.I + A.first + blockIdx.x / t.size, sizeof I);
+    if (tid < 2 * kSolveMaxCluster) (&slot[0][0])[tid] = 0.0;
+    if (tid < kSolveWarps) warp_sums[tid] = 0.0;
     __syncthreads();
     IScal &S = G.S[I.inst];
     // (read by every CTA before its first team barrier, written after the last)
@@ -294,201 +356,217 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_solve(PcgFine G, SolveArgs
     const double tol2 = S.tol2;
     double tol2in = S.tol2in, rr = S.rr;
     int status = 0, iters = 0, iters_prev = 0, outer = 0;
-    const int n = I.n, s0 = I.s, clev = I.clev;
+    const int n = I.n, clev = I.clev;
     for (int k = tid; k < kSolveVecs * t.size; k += nt) rng[k / t.size][k % t.size] = I.rng[k];
+    copy4(&Rk, I.ranks + t.rank, sizeof Rk);
     __syncthreads();
 
-    // ---- shared memory: tables, row descriptors, vectors
-    auto copy16 = [&](uint32_t to, const void *from, uint32_t bytes) {
-        for (uint32_t k = tid; k < bytes / 16; k += nt)
-            reinterpret_cast<uint4 *>(dyn + to)[k] = __ldg(reinterpret_cast<const uint4 *>(from) + k);
+    // ---- shared memory: operators, descriptors, vectors
+    const char *rt = I.rank_tables;
+    auto load = [&](const STab &b, const char *from) {
+        if (b.s == kSolveGlobal) return;
+        for (uint32_t k = tid; k < b.bytes / 16; k += nt)
+            at<uint4>(b.s + 16 * k) = __ldg(reinterpret_cast<const uint4 *>(from + b.g) + k);
     };
-    auto load_tab = [&](const STab &b) { if (b.s != kSolveGlobal) copy16(b.s, I.tables + b.g, b.bytes); };
-    auto table = [&](const STab &b) -> const char * { return b.s != kSolveGlobal ? dyn + b.s : I.tables + b.g; };
-    auto ents = [&](const STab &b) { return reinterpret_cast<const SEnt<T> *>(table(b)); };
-    load_tab(I.a);
-    load_tab(I.inv);
-    if (MIX) load_tab(I.a64);
-    T *tail = reinterpret_cast<T *>(dyn);
-    auto vec = [&](int id, T *sh, T *global, int lo, int hi) {
+    load(I.a, I.tables);
+    load(I.m, I.tables);
+    load(I.inv, I.tables);
+    load(I.tpv, I.tables);
+    load(I.tpo, I.tables);
+    load(I.trv, I.tables);
+    load(I.tro, I.tables);
+    load(Rk.desc0, rt);
+    load(Rk.desc_r, rt);
+    for (int l = 0; l < clev; l++) {
+        load(Rk.down[l].t, rt);
+        load(Rk.up[l].t, rt);
+    }
+    auto vec = [&](int id, uint32_t off, int rows) {
         solve::Vec<T> v;
         const int4 g = rng[id][t.rank];
-        v.sh = sh;
-        v.at = sh ? sh - g.x : global;
+        int lo, hi;
+        solve::rank_rows(t.rank, t.size, rows, lo, hi);
+        v.base = off - (uint32_t)g.x * kT;
+        v.sh = solve::address(solve::dyn + off);
         v.rng = rng[id];
         v.rank = t.rank;
         v.klo = g.z;
         v.khi = g.w;
+        // rows that some other rank holds too: below own_lo, from own_hi
         v.own_lo = lo;
         v.own_hi = hi;
-        if (sh && t.size > 1) {
-            // rows that some other rank holds too: below own_lo, from own_hi
-            for (int k = g.z; k < t.rank; k++) v.own_lo = max(v.own_lo, min(hi, rng[id][k].y));
-            for (int k = t.rank + 1; k <= g.w; k++) v.own_hi = min(v.own_hi, max(lo, rng[id][k].x));
-        }
+        for (int k = g.z; k < t.rank; k++) v.own_lo = max(v.own_lo, min(hi, rng[id][k].y));
+        for (int k = t.rank + 1; k <= g.w; k++) v.own_hi = min(v.own_hi, max(lo, rng[id][k].x));
         return v;
     };
+    auto resolve = [&](const SOp &o) {
+        const uint32_t b = o.t.s != kSolveGlobal ? o.t.s : 0u;
+        return solve::Op{o.t.s != kSolveGlobal ? nullptr : rt + o.t.g, b, b + o.val, b + o.idx, o.row0, o.rows, o.lg, o.nsl};
+    };
+    if (tid < clev) {
+        od[tid] = resolve(Rk.down[tid]);
+        ou[tid] = resolve(Rk.up[tid]);
+        if (tid > 0) {
+            vb[tid] = vec(2 * tid, I.vb[tid], I.lvl[tid]);
+            vo[tid] = vec(2 * tid + 1, I.vo[tid], I.lvl[tid]);
+        }
+    }
     int lo, hi;
     solve::rank_rows(t.rank, t.size, n, lo, hi);
-    auto log2i = [](int v) { return 31 - __clz(v); };
-    for (int l = 0; l < max(1, clev); l++) {
-        const SLevel &L = I.L[l];
-        load_tab(L.r);
-        load_tab(L.m);
-        load_tab(L.p);
-        // row descriptors: of the own rows (above the tail), or all
-        const int nr = l + 1 < clev ? I.L[l + 1].n : clev > 0 ? I.nc : 0;
-        int a = 0, h = nr, ua = 0, uh = L.n;
-        if (l < s0 || clev == 0) {
-            solve::rank_rows(t.rank, t.size, nr, a, h);
-            solve::rank_rows(t.rank, t.size, L.n, ua, uh);
-        }
-        if (L.srow_u != kSolveGlobal)
-            for (int i = ua + tid; i < uh; i += nt)
-                reinterpret_cast<uint4 *>(dyn + L.srow_u)[i - ua] = __ldg(I.rows_u + L.row_u + i);
-        if (L.srow_r != kSolveGlobal)
-            for (int i = a + tid; i < h; i += nt)
-                reinterpret_cast<uint2 *>(dyn + L.srow_r)[i - a] = __ldg(I.rows_r + L.row_r + i);
-        if (tid == 0) {
-            solve::Plan<T> &P = plan[l];
-            P.tr = ents(L.r);
-            P.tm = ents(L.m);
-            P.tp = ents(L.p);
-            P.rr = L.srow_r != kSolveGlobal ? reinterpret_cast<const uint2 *>(dyn + L.srow_r) - a : I.rows_r + L.row_r;
-            P.ru = L.srow_u != kSolveGlobal ? reinterpret_cast<const uint4 *>(dyn + L.srow_u) - ua : I.rows_u + L.row_u;
-            P.rlo = a;
-            P.rhi = h;
-            P.ulo = ua;
-            P.uhi = uh;
-            P.lr = log2i(L.lanes_r);
-            P.lu = log2i(L.lanes_u);
-            if (l == 0) {
-                P.b = vec(0, I.vr == kSolveGlobal ? nullptr : reinterpret_cast<T *>(dyn + I.vr), A.r + I.row0, ua, uh);
-                P.o = vec(1, I.vz == kSolveGlobal ? nullptr : reinterpret_cast<T *>(dyn + I.vz), A.z + I.row0, ua, uh);
-            } else if (l < s0) {
-                P.b = vec(2 * l, L.vb == kSolveGlobal ? nullptr : tail + L.vb, I.gvec + L.gb, ua, uh);
-                P.o = vec(2 * l + 1, L.vo == kSolveGlobal ? nullptr : tail + L.vo, I.gvec + L.go, ua, uh);
-            } else {
-                P.b.at = tail + L.vb;
-                P.o.at = tail + L.vo;
-            }
-        }
-    }
-    __syncthreads();
-    const solve::Plan<T> &P0 = plan[0];
-    const solve::Vec<T> r = P0.b, z = P0.o;
+    const solve::Vec<T> r = vec(0, I.vr, n), q = vec(0, I.vq, n), z = vec(1, I.vz, n);
+    const int xlo = rng[0][t.rank].x, xhi = rng[0][t.rank].y;   // rows held of r and q
     // own rows only
-    auto priv = [&](uint32_t off, T *global) { return off == kSolveGlobal ? global : reinterpret_cast<T *>(dyn + off) - lo; };
-    T *p = priv(I.vp, A.p + I.row0), *q = priv(I.vq, A.q + I.row0);
-    T *e = MIX ? priv(I.vx, A.e + I.row0) : nullptr;
+    const bool ps = I.vp != kSolveGlobal, xs = I.vx != kSolveGlobal;
+    T *pg = A.p + I.row0, *eg = MIX ? A.e + I.row0 : nullptr;
+    const uint32_t pb = I.vp - (uint32_t)lo * kT, xb = I.vx - (uint32_t)lo * (MIX ? kT : 8u);
     const int pt = G.projtype_all >= 0 ? G.projtype_all : G.ipar[I.inst].projtype;
     double *xg = (pt == HF_INCREMENTAL ? G.dp : G.p) + I.row0;
-    double *x = !MIX && I.vx != kSolveGlobal ? reinterpret_cast<double *>(dyn + I.vx) - lo : xg;
-    if (x != xg)
-        for (int i = lo + tid; i < hi; i += nt) x[i] = xg[i];
-    if (I.vr != kSolveGlobal) {
-        const int4 g = rng[0][t.rank];
-        for (int i = g.x + tid; i < g.y; i += nt) r.at[i] = A.r[I.row0 + i];
-    }
-    const SEnt<T> *tabA = ents(I.a), *tabM = P0.tm;
-    const uint4 *rows0 = P0.ru;
+    if (!MIX && xs)
+        for (int i = lo + tid; i < hi; i += nt) at<double>(xb + 8u * i) = xg[i];
+    for (int i = xlo + tid; i < xhi; i += nt) at<T>(r.row(i)) = A.r[I.row0 + i];
+    const uint32_t tabA = I.a.s, tabM = I.m.s, desc = Rk.desc0.s - 8u * (uint32_t)lo;
+    const int kk = K > 0 ? K : kf;
+    const uint32_t cb = I.cvec, co = cb + (uint32_t)I.nc * kT, cb_sh = solve::address(solve::dyn + cb);
+    // the first way down in template form: own rows
+    int ra, rh;
+    solve::rank_rows(t.rank, t.size, clev == 1 ? I.nc : clev > 1 ? I.lvl[1] : 0, ra, rh);
+    const uint32_t desc_r = Rk.desc_r.s - 8u * (uint32_t)ra;
+    const bool tpl_p = I.tpl_p != 0, tpl_r = I.tpl_r != 0;
+    const uint32_t tpv = I.tpv.s, tpo = I.tpo.s, trv = I.trv.s, tro = I.tro.s;
+    const int lg_r = I.lg_r;
+    int lg_d = 5;   // threads per row of the dense solve (log2)
+    while (lg_d > 0 && (I.nc << lg_d) > nt) lg_d--;
     // every CTA of the cluster has started (its shared memory may be written)
     solve::team_sync(t);
 
-    // the dense solve of the coarsest level
-    const T *inv = reinterpret_cast<const T *>(table(I.inv));
-    T *cb = tail + I.cvec, *co = cb + I.nc;
+    // the dense solve of the coarsest level, every CTA for itself
     auto dense = [&]() {
-        const int nc = I.nc;
-        int lg = 5;
-        while (lg > 0 && (nc << lg) > nt) lg--;
-        const int lanes = 1 << lg, lane = tid & (lanes - 1), step = nt >> lg;
-        for (int base = 0; base < nc; base += step) {
-            const int i = base + (tid >> lg);
+        const int nc = I.nc, lanes = 1 << lg_d, lane = tid & (lanes - 1), step = nt >> lg_d;
+        const uint32_t is = I.inv.s;
+        for (int b = 0; b < nc; b += step) {
+            const int i = b + (tid >> lg_d);
             T s = T(0);
             if (i < nc) {
-                const T *row = inv + (size_t)i * nc;
+                if (is != kSolveGlobal) {
+                    const uint32_t row = is + (uint32_t)(i * nc) * kT;
 #pragma unroll 4
-                for (int k = lane; k < nc; k += lanes) s = solve::fma_(row[k], cb[k], s);
+                    for (int k = lane; k < nc; k += lanes) s = solve::fma_(at<T>(row + k * kT), at<T>(cb + k * kT), s);
+                } else {
+                    const T *row = reinterpret_cast<const T *>(I.tables + I.inv.g) + (size_t)i * nc;
+#pragma unroll 4
+                    for (int k = lane; k < nc; k += lanes) s = solve::fma_(__ldg(row + k), at<T>(cb + k * kT), s);
+                }
             }
             s = solve::lanes_sum(s, lanes);
-            if (i < nc && lane == 0) co[i] = s;
+            if (i < nc && lane == 0) at<T>(co + i * kT) = s;
         }
         __syncthreads();
     };
-
-    // z = V-cycle of r; returns this thread's part of r.z (the team has not
-    // yet met on z)
-    auto vcycle = [&]() -> double {
-        double part = 0.0;
+    // rows of the coarsest level: to every CTA
+    auto to_all = [&](int i, T v, int lane, int lanes) {
+        if (t.size > 1) {
+            for (int k = lane; k < t.size; k += lanes) solve::store_peer(solve::peer(cb_sh + i * kT, k), v);
+        } else if (lane == 0) {
+            at<T>(cb + i * kT) = v;
+        }
+    };
+    // the way down from level l: b_{l+1} = Rt b_l
+    auto down = [&](int l) {
+        const bool last = l + 1 == clev;
+        const solve::Vec<T> nb = vb[last ? l : l + 1];
+        const int lg = od[l].lg;
+        solve::apply<T>(od[l], [&](int i, T v, int lane) {
+            if (last) to_all(i, v, lane, 1 << lg);
+            else if (lane == 0) nb.put(i, v);
+        });
+    };
+    auto first_down = [&]() {
         if (clev == 0) {
             // the finest level is the coarsest: one CTA
-            for (int i = tid; i < n; i += nt) cb[i] = r.at[i];
-            __syncthreads();
-            dense();
-            for (int i = lo + tid; i < hi; i += nt) {
-                z.put(i, co[i]);
-                part += (double)r.at[i] * (double)co[i];
-            }
-            return part;
+            for (int i = tid; i < n; i += nt) at<T>(cb + i * kT) = r.get(i);
+            return;
         }
-        // down the distributed levels
-        for (int l = 0; l < s0; l++) {
-            const solve::Plan<T> &P = plan[l];
-            if (l + 1 == s0) {
-                // the tail's rows: to every CTA
-                T *nb = l + 1 == clev ? cb : plan[l + 1].b.at;
-                solve::down(P, (const T *)P.b.at, [&](int i, T v, int lane) {
-                    if (t.size > 1) {
-                        for (int k = lane; k < t.size; k += 1 << P.lr) cg::this_cluster().map_shared_rank(nb, k)[i] = v;
-                    } else if (lane == 0) {
-                        nb[i] = v;
-                    }
-                });
-            } else {
-                const solve::Vec<T> &nb = plan[l + 1].b;
-                solve::down(P, (const T *)P.b.at, [&](int i, T v, int lane) { if (lane == 0) nb.put(i, v); });
+        if (!tpl_r) {
+            down(0);
+            return;
+        }
+        const bool last = clev == 1;
+        const solve::Vec<T> nb = vb[1];
+        const int lanes = 1 << lg_r, lane = tid & (lanes - 1), step = nt >> lg_r;
+        for (int b = ra; b < rh; b += step) {
+            const int i = b + (tid >> lg_r);
+            const uint2 d = i < rh ? at<uint2>(desc_r + 8u * i) : make_uint2(0u, 0u);
+            const T s = solve::lanes_sum(solve::row_part<T>(trv, tro, d.x, lane, lanes, d.y * kT), lanes);
+            if (i < rh) {
+                if (last) to_all(i, s, lane, lanes);
+                else if (lane == 0) nb.put(i, s);
             }
+        }
+    };
+    // the V-cycle's rest: z, and this thread's part of r.z (the team has met on
+    // b_1, and has not yet on z)
+    auto vcycle = [&]() -> double {
+        double part = 0.0;
+        for (int l = 1; l < clev; l++) {
+            down(l);
             solve::team_sync(t);
-        }
-        // the tail, every CTA for itself
-        for (int l = s0; l < clev; l++) {
-            const solve::Plan<T> &P = plan[l];
-            T *nb = l + 1 == clev ? cb : plan[l + 1].b.at;
-            solve::down(P, (const T *)P.b.at, [&](int i, T v, int lane) { if (lane == 0) nb[i] = v; });
-            __syncthreads();
         }
         dense();
-        const T *ev = co;
-        for (int l = clev - 1; l >= s0; l--) {
-            const solve::Plan<T> &P = plan[l];
-            T *ol = P.o.at;
-            solve::up(P, (const T *)P.b.at, ev, [&](int i, T v) { ol[i] = v; });
-            __syncthreads();
-            ev = ol;
-        }
-        // up the distributed levels
-        for (int l = s0 - 1; l > 0; l--) {
-            const solve::Plan<T> &P = plan[l];
-            solve::up(P, (const T *)P.b.at, ev, [&](int i, T v) { P.o.put(i, v); });
+        for (int l = clev - 1; l > 0; l--) {
+            const solve::Vec<T> ol = vo[l];
+            solve::apply<T>(ou[l], [&](int i, T v, int lane) { if (lane == 0) ol.put(i, v); });
             solve::team_sync(t);
-            ev = P.o.at;
         }
-        const SEnt<T> *tp = P0.tp;
-        for (int i = lo + tid; i < hi; i += nt) {
-            const uint4 d = rows0[i];
-            const T v = solve::fine_row<K>(tabM, d.x, (const T *)(r.at + i)) + solve::row_part(tp, d.y, 0, 1, ev + (int)d.z);
-            z.put(i, v);
-            part += (double)r.at[i] * (double)v;
+        if (clev == 0) {
+            for (int i = lo + tid; i < hi; i += nt) {
+                const T v = at<T>(co + i * kT);
+                z.put(i, v);
+                part += (double)r.get(i) * (double)v;
+            }
+        } else if (tpl_p) {
+            for (int i = lo + tid; i < hi; i += nt) {
+                const uint2 d = at<uint2>(desc + 8u * i);
+                const T v = solve::row_fixed<K, T>(tabM + (d.y & 0xffffu) * kk * kE, kk, r.row(i)) +
+                            solve::row_part<T>(tpv, tpo, d.x, 0, 1, (d.y >> 16) * kT);
+                z.put(i, v);
+                part += (double)r.get(i) * (double)v;
+            }
+        } else {
+            const solve::Op P = ou[0];
+            for (int k = tid >> 5; k < P.nsl; k += nt >> 5) {
+                const int i = lo + 32 * k + (tid & 31);
+                T v = solve::slice_part<T>(P, k);
+                if (i < hi) {
+                    v += solve::row_fixed<K, T>(tabM + (at<uint2>(desc + 8u * i).y & 0xffffu) * kk * kE, kk, r.row(i));
+                    z.put(i, v);
+                    part += (double)r.get(i) * (double)v;
+                }
+            }
         }
         return part;
     };
 
     for (int sweep = 0;; sweep++) {
-        double rz = 0.0;
+        double rz = 0.0, part = 0.0;
         iters = 0;
-        bool inner = true;
-        while (inner) {
+        while (true) {
+            first_down();
+            if (iters == 0) {
+                solve::team_sync(t);
+            } else {
+                // ||r|| of the last update
+                const double tot = solve::team_sum(t, part);
+                if (!MIX) rr = tot;
+                if (!isfinite(tot)) {
+                    status = HF_ERR_NAN;
+                    break;
+                }
+                if (!(tot > (MIX ? tol2in : tol2))) break;
+                if (MIX ? (iters >= G.inner_maxit || iters + iters_prev >= G.maxit) : iters >= G.maxit) {
+                    if (!MIX) status = HF_ERR_NOT_CONVERGED;
+                    break;
+                }
+            }
             double tot = solve::team_sum(t, vcycle());
             const bool first = iters == 0;
             const T beta = first ? T(0) : T(tot / rz);
@@ -498,14 +576,17 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_solve(PcgFine G, SolveArgs
                 break;
             }
             // p = z + beta p, q = A z + beta q
-            double part = 0.0;
+            part = 0.0;
             for (int i = lo + tid; i < hi; i += nt) {
-                const T w = solve::fine_row<K>(tabA, rows0[i].x, (const T *)(z.at + i));
-                const T zi = z.at[i];
-                const T pi = first ? zi : solve::fma_(beta, p[i], zi);
-                const T qi = first ? w : solve::fma_(beta, q[i], w);
-                p[i] = pi;
-                q[i] = qi;
+                const T w = solve::row_fixed<K, T>(tabA + (at<uint2>(desc + 8u * i).y & 0xffffu) * kk * kE, kk, z.row(i));
+                T pi = z.get(i), qi = w;
+                if (!first) {
+                    pi = solve::fma_(beta, ps ? at<T>(pb + i * kT) : pg[i], pi);
+                    qi = solve::fma_(beta, q.get(i), w);
+                }
+                if (ps) at<T>(pb + i * kT) = pi;
+                else pg[i] = pi;
+                q.put(i, qi);
                 part += (double)pi * (double)qi;
             }
             tot = solve::team_sum(t, part);
@@ -523,51 +604,45 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_solve(PcgFine G, SolveArgs
             const double alpha = rz / tot;
             const T al = (T)alpha;
             part = 0.0;
-            for (int i = lo + tid; i < hi; i += nt) {
-                const T pi = p[i];
-                const T ri = solve::fma_(-al, q[i], r.at[i]);
-                r.put(i, ri);
+            for (int i = xlo + tid; i < xhi; i += nt) {
+                const T ri = solve::fma_(-al, q.get(i), r.get(i));
+                at<T>(r.row(i)) = ri;
+                if (i < lo || i >= hi) continue;   // the halo
+                const T pi = ps ? at<T>(pb + i * kT) : pg[i];
                 part += (double)ri * (double)ri;
-                if (MIX) e[i] = first ? al * pi : solve::fma_(al, pi, e[i]);
-                else x[i] = __fma_rn(alpha, (double)pi, x[i]);
+                if (MIX) {
+                    T v = al * pi;
+                    if (!first) v = solve::fma_(al, pi, xs ? at<T>(xb + i * kT) : eg[i]);
+                    if (xs) at<T>(xb + i * kT) = v;
+                    else eg[i] = v;
+                } else if (xs) {
+                    at<double>(xb + 8u * i) = __fma_rn(alpha, (double)pi, at<double>(xb + 8u * i));
+                } else {
+                    xg[i] = __fma_rn(alpha, (double)pi, xg[i]);
+                }
             }
-            tot = solve::team_sum(t, part);
             iters++;
-            if (!MIX) rr = tot;
-            if (!isfinite(tot)) {
-                status = HF_ERR_NAN;
-                inner = false;
-            } else if (!(tot > (MIX ? tol2in : tol2))) {
-                inner = false;
-            } else if (MIX ? (iters >= G.inner_maxit || iters + iters_prev >= G.maxit) : iters >= G.maxit) {
-                if (!MIX) status = HF_ERR_NOT_CONVERGED;
-                inner = false;
-            }
+            __syncthreads();
         }
         if (!MIX) break;
         // the FP64 refinement step (k_ir_correct): x += e, r -= A e, ||r||
         // against the plain form's target; e takes z's place, with its halo
         double *r64 = G.r + I.row0;
-        const SEnt<double> *tab64 = reinterpret_cast<const SEnt<double> *>(table(I.a64));
+        const SEnt<double> *tab64 = reinterpret_cast<const SEnt<double> *>(I.tables + I.a64.g);
         // (a sweep that ended before its first update has no correction)
         const bool apply = status == 0 && iters > 0;
         if (apply) {
-            for (int i = lo + tid; i < hi; i += nt) z.put(i, e[i]);
+            for (int i = lo + tid; i < hi; i += nt) z.put(i, xs ? at<T>(xb + i * kT) : eg[i]);
             solve::team_sync(t);
         }
-        double part = 0.0;
+        part = 0.0;
         for (int i = lo + tid; i < hi; i += nt) {
             double ri = r64[i];
             if (apply) {
-                const uint32_t d = rows0[i].x;
-                const SEnt<double> *te = tab64 + (d >> kSolveLenBits);
-                const int len = (int)(d & ((1u << kSolveLenBits) - 1));
+                const SEnt<double> *te = tab64 + (at<uint2>(desc + 8u * i).y & 0xffffu) * kk;
                 double ax = 0.0;
-                for (int k = 0; k < len; k++) {
-                    const SEnt<double> a = te[k];
-                    ax += a.v * (double)z.at[i + a.off];
-                }
-                x[i] += (double)e[i];
+                for (int k = 0; k < kk; k++) ax += __ldg(&te[k].v) * (double)z.get(i + __ldg(&te[k].off));
+                xg[i] += (double)z.get(i);
                 ri -= ax;
                 r64[i] = ri;
                 r.put(i, (T)ri);
@@ -589,8 +664,8 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_solve(PcgFine G, SolveArgs
         iters_prev += iters;
         tol2in = fmax(tol2, G.eta * G.eta * rr);
     }
-    if (x != xg)
-        for (int i = lo + tid; i < hi; i += nt) xg[i] = x[i];
+    if (!MIX && xs)
+        for (int i = lo + tid; i < hi; i += nt) xg[i] = at<double>(xb + 8u * i);
     if (tid == 0 && t.rank == 0) {
         S.rr = rr;
         S.iters = iters;
@@ -606,7 +681,7 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_solve(PcgFine G, SolveArgs
 }
 
 // ---------------------------------------------------------------------------
-// host: the folded operators of one instance as row templates
+// host: the folded operators of one instance
 // ---------------------------------------------------------------------------
 namespace solve {
 
@@ -616,7 +691,6 @@ namespace solve {
 // that is set).
 struct Tables {
     int pad = 1, fixed = 0;
-    std::vector<uint32_t> desc;
     std::vector<int32_t> off;
     std::vector<double> v, v2;
     std::unordered_map<std::string, uint32_t> seen;
@@ -640,48 +714,75 @@ struct Tables {
         }
         const uint32_t d = ((uint32_t)off.size() << kSolveLenBits) | (uint32_t)full;
         seen.emplace(key, d);
-        for (int k = 0; k < len; k++) {
-            off.push_back(col[k] - anchor);
-            v.push_back(val[k]);
-            if (val2) v2.push_back(val2[k]);
-        }
-        for (int k = len; k < full; k++) {
-            off.push_back(len ? col[len - 1] - anchor : 0);
-            v.push_back(0.0);
-            if (val2) v2.push_back(0.0);
+        for (int k = 0; k < full; k++) {
+            off.push_back(k < len ? col[k] - anchor : len ? col[len - 1] - anchor : 0);
+            v.push_back(k < len ? val[k] : 0.0);
+            if (val2) v2.push_back(k < len ? val2[k] : 0.0);
         }
         return d;
     }
 };
 
+// sparse rows of one folded operator
+struct Csr {
+    std::vector<int> ptr{0}, col;
+    std::vector<double> val;
+    void add(int c, double v)
+    {
+        if (v == 0.0) return;
+        col.push_back(c);
+        val.push_back(v);
+    }
+    void end_row() { ptr.push_back((int)col.size()); }
+    int rows() const { return (int)ptr.size() - 1; }
+};
+
+// row i of A as row rpos[i], its columns c as cpos[c] (empty: unchanged), sorted
+inline Csr permuted(const Csr &A, const std::vector<int> &rpos, const std::vector<int> &cpos)
+{
+    const int n = A.rows();
+    std::vector<int> at(n);
+    for (int i = 0; i < n; i++) at[rpos.empty() ? i : rpos[i]] = i;
+    Csr B;
+    B.col.reserve(A.col.size());
+    B.val.reserve(A.val.size());
+    std::vector<std::pair<int, double>> row;
+    for (int j = 0; j < n; j++) {
+        row.clear();
+        for (int k = A.ptr[at[j]]; k < A.ptr[at[j] + 1]; k++)
+            row.emplace_back(cpos.empty() ? A.col[k] : cpos[A.col[k]], A.val[k]);
+        std::sort(row.begin(), row.end(), [](const auto &a, const auto &b) { return a.first < b.first; });
+        for (const auto &e : row) {
+            B.col.push_back(e.first);
+            B.val.push_back(e.second);
+        }
+        B.end_row();
+    }
+    return B;
+}
+
 struct HostSolve {
     bool ok = false;
-    int s = 0, clev = 0, nc = 0, cluster = 1, fine = 0;   // fine: k_solve's K
+    int clev = 0, nc = 0, cluster = 1, threads = 256, fine = 0;   // fine: entries of the finest operator's rows
     std::vector<int4> rng;      // [kSolveVecs][cluster], see SInst::rng
     int held[kSolveVecs] = {};  // most rows a rank holds of the vector
     struct Level {
-        int n = 0, lanes_r = 1, lanes_u = 1;
-        std::vector<uint2> rows_r;
-        std::vector<uint4> rows_u;
-        std::vector<int32_t> off_r, off_m, off_p;
-        std::vector<double> v_r, v_m, v_p, v_a;   // v_a: the finest operator on off_m's pattern
+        int n = 0;
+        Csr m, p, r;            // Mt (levels above 0), Pt, Rt
     };
     std::vector<Level> L;
+    std::vector<int> cpos;      // the coarsest level's rows: their places here (empty: unchanged)
+    // finest level: A and Mt as templates of `fine` entries, per row the template
+    std::vector<uint32_t> tpl;
+    std::vector<int32_t> off;
+    std::vector<double> va, vm;
 };
-
-inline int lanes_for(double avg)
-{
-    int l = 1;
-    while (l < 32 && avg > 12.0 * l) l *= 2;
-    return l;
-}
 
 // CTAs of an instance's cluster: about kSolveRows rows each while the case's
 // instances leave SMs idle (a phase then takes one row per thread or less and
-// the barriers dominate), up to 4096 when they fill the device anyway.
-// Measured, Poisson solve per step: 4,096 rows alone (FP64) 218 / 232 / 269 /
-// 311 / 383 us at 256 / 512 / 1024 / 2048 / 4096 rows a CTA; 32 instances with
-// 515,000 rows (mixed) 1785 / 1540 / 1354 / 1310 us at 512 / 1024 / 2048 / 4096.
+// its latency counts), up to 4096 when they fill the device anyway.  Measured,
+// Poisson solve per step: 4,096 rows alone (FP64) 150 / 148 / 170 / 255 us at
+// 256 / 512 / 1024 / 2048 rows a CTA, 4,913 rows in 3D 209 / 210 / 273 / 354.
 constexpr int kSolveRows = 512;
 inline int cluster_size(int n, long total)
 {
@@ -692,6 +793,17 @@ inline int cluster_size(int n, long total)
     return c;
 }
 
+// Threads of a CTA with `own` rows of the finest level: the fewest turns a full
+// block needs, and no more warps than these turns take (every warp pays a
+// phase's fixed instructions).  The instances of a batch share three sizes, so
+// that few launches cover them.
+inline int block_threads(int own, bool batch)
+{
+    if (batch) return own <= 256 ? 256 : own <= 512 ? 512 : kSolveThreads;
+    const int turns = (own + kSolveThreads - 1) / kSolveThreads;
+    return std::min(kSolveThreads, std::max(128, ((own + turns - 1) / turns + 31) / 32 * 32));
+}
+
 // the rows of every vector that each rank holds: its own and the columns its
 // rows reach
 inline void ranges(HostSolve &S)
@@ -699,15 +811,18 @@ inline void ranges(HostSolve &S)
     const int C = S.cluster;
     S.rng.assign((size_t)kSolveVecs * C, make_int4(0, 0, 0, 0));
     auto rows = [&](int l) { return l < (int)S.L.size() ? S.L[l].n : S.nc; };
-    auto grow = [](int4 &g, int lo, int hi) {
-        g.x = std::min(g.x, lo);
-        g.y = std::max(g.y, hi);
+    auto grow = [](int4 &g, int c) {
+        g.x = std::min(g.x, c);
+        g.y = std::max(g.y, c + 1);
     };
-    auto reach = [&](int4 &g, const std::vector<int32_t> &off, uint32_t d, int anchor) {
-        for (uint32_t k = d >> kSolveLenBits, e = k + (d & ((1u << kSolveLenBits) - 1)); k < e; k++)
-            grow(g, anchor + off[k], anchor + off[k] + 1);
+    auto reach = [&](int4 &g, const Csr &A, int lo, int hi) {
+        for (int k = A.ptr[lo]; k < A.ptr[hi]; k++) grow(g, A.col[k]);
     };
-    const int levels = std::max(1, S.s);   // levels with distributed vectors
+    auto reach_fine = [&](int4 &g, int lo, int hi) {
+        for (int i = lo; i < hi; i++)
+            for (int k = 0; k < S.fine; k++) grow(g, i + S.off[(size_t)S.tpl[i] * S.fine + k]);
+    };
+    const int levels = std::max(1, S.clev);   // levels with distributed vectors
     for (int l = 0; l < levels; l++) {
         const HostSolve::Level &L = S.L[l];
         for (int k = 0; k < C; k++) {
@@ -716,21 +831,22 @@ inline void ranges(HostSolve &S)
             // b of the level (the residual on the finest): Mt and Rt rows
             int4 &b = S.rng[(size_t)(2 * l) * C + k];
             b = make_int4(lo, hi, k, k);
-            for (int i = lo; i < hi; i++) reach(b, L.off_m, L.rows_u[i].x, i);
+            if (l == 0) reach_fine(b, lo, hi);
+            else reach(b, L.m, lo, hi);
             if (l < S.clev) {
                 rank_rows(k, C, rows(l + 1), a, h);
-                for (int i = a; i < h; i++) reach(b, L.off_r, L.rows_r[i].x, (int)L.rows_r[i].y);
+                reach(b, L.r, a, h);
             }
-            // z on the finest level: A rows (Mt's pattern); out of a level
-            // between: the Pt rows of the level above
+            // z on the finest level: A rows; out of a level between: the Pt
+            // rows of the level above
             int4 &o = S.rng[(size_t)(2 * l + 1) * C + k];
             o = make_int4(lo, hi, k, k);
             if (l == 0) {
-                for (int i = lo; i < hi; i++) reach(o, L.off_m, L.rows_u[i].x, i);
+                reach_fine(o, lo, hi);
             } else {
                 const HostSolve::Level &F = S.L[l - 1];
                 rank_rows(k, C, F.n, a, h);
-                for (int i = a; i < h; i++) reach(o, F.off_p, F.rows_u[i].y, (int)F.rows_u[i].z);
+                reach(o, F.p, a, h);
             }
         }
     }
@@ -755,100 +871,372 @@ inline HostSolve build(const std::vector<hf::HostLevel> &H, long total)
     HostSolve S;
     S.clev = (int)H.size() - 1;
     S.nc = H.back().A.n;
-    S.s = S.clev == 0 ? 0 : 1;
-    while (S.s < S.clev && H[S.s].A.n > kSolveTail) S.s++;
     if (S.nc > kCoarseCap || S.clev >= kMaxLevels) return S;
-    size_t tail = 2 * S.nc;   // the tail's vectors always live in shared memory
-    for (int l = std::max(1, S.s); l < S.clev; l++) tail += 2 * H[l].A.n;
-    if (tail * sizeof(double) > kSolveSmem / 2) return S;
     S.cluster = S.clev == 0 ? 1 : cluster_size(H[0].A.n, total);
+    S.threads = block_threads((H[0].A.n + S.cluster - 1) / S.cluster, total > H[0].A.n);
     S.L.resize(std::max(1, S.clev));
     for (int l = 0; l < (int)S.L.size(); l++) {
         const hf::HostLevel &h = H[l];
         HostSolve::Level &o = S.L[l];
         const int n = h.A.n;
         o.n = n;
-        o.rows_u.resize(n);
         std::vector<double> d(n);
         for (int i = 0; i < n; i++) d[i] = h.omega * h.dinv[i];
-        Tables tm, tp, tr;
-        o.lanes_r = l < S.clev ? lanes_for((double)h.R.ptr[h.R.n] / std::max(1, h.R.n) * 1.9) : 1;
-        o.lanes_u = l == 0 ? 1 : lanes_for((double)h.A.ptr[n] / n * 0.75);
-        tr.pad = 2 * o.lanes_r;
-        tm.pad = tp.pad = 2 * o.lanes_u;
         if (l == 0) {
-            int most = 0;
+            int most = 1;
             for (int i = 0; i < n; i++) most = std::max(most, h.A.ptr[i + 1] - h.A.ptr[i]);
-            S.fine = tm.fixed = most <= 5 ? 5 : most <= 7 ? 7 : 0;
-        }
-        std::vector<double> mv;
-        for (int i = 0; i < n; i++) {
-            const int a = h.A.ptr[i], len = h.A.ptr[i + 1] - a;
-            mv.resize(len);
-            for (int k = 0; k < len; k++) {
-                const int j = h.A.col[a + k];
-                mv[k] = (j == i ? 2.0 * d[i] : 0.0) - d[i] * h.A.val[a + k] * d[j];
+            Tables tm;
+            S.fine = tm.fixed = most <= 5 ? 5 : most <= 7 ? 7 : most;
+            S.tpl.resize(n);
+            std::vector<double> mv;
+            for (int i = 0; i < n; i++) {
+                const int a = h.A.ptr[i], len = h.A.ptr[i + 1] - a;
+                mv.resize(len);
+                for (int k = 0; k < len; k++) {
+                    const int j = h.A.col[a + k];
+                    mv[k] = (j == i ? 2.0 * d[i] : 0.0) - d[i] * h.A.val[a + k] * d[j];
+                }
+                S.tpl[i] = (tm.row(&h.A.col[a], mv.data(), &h.A.val[a], len, i) >> kSolveLenBits) / S.fine;
+                if (S.tpl[i] > 0xffffu) tm.ok = false;
+                if (!tm.ok) return S;
             }
-            const uint32_t ds = tm.row(&h.A.col[a], mv.data(), l == 0 ? &h.A.val[a] : nullptr, len, i);
-            o.rows_u[i] = make_uint4(ds, 0u, 0u, 0u);
+            S.off = std::move(tm.off);
+            S.vm = std::move(tm.v);
+            S.va = std::move(tm.v2);
+        } else {
+            for (int i = 0; i < n; i++) {
+                for (int k = h.A.ptr[i]; k < h.A.ptr[i + 1]; k++) {
+                    const int j = h.A.col[k];
+                    o.m.add(j, (j == i ? 2.0 * d[i] : 0.0) - d[i] * h.A.val[k] * d[j]);
+                }
+                o.m.end_row();
+            }
         }
-        o.off_m = std::move(tm.off);
-        o.v_m = std::move(tm.v);
-        o.v_a = std::move(tm.v2);
-        if (!tm.ok) return S;
-        if (l >= S.clev) {   // the finest level is the coarsest: its operator only
-            ranges(S);
-            S.ok = true;
-            return S;
-        }
+        if (l >= S.clev) break;   // the finest level is the coarsest
         // Pt = P - w D^-1 A P
         hf::HostCSR AP = hf::csr_multiply(h.A, h.P);
-        std::vector<int> col;
-        std::vector<double> val, acc(std::max(h.P.m, n), 0.0);
+        std::vector<double> acc(std::max(h.P.m, n), 0.0);
         for (int i = 0; i < n; i++) {
             for (int k = h.P.ptr[i]; k < h.P.ptr[i + 1]; k++) acc[h.P.col[k]] = h.P.val[k];
-            col.clear();
-            val.clear();
-            for (int k = AP.ptr[i]; k < AP.ptr[i + 1]; k++) {
-                const double v = acc[AP.col[k]] - d[i] * AP.val[k];
-                if (v != 0.0) {
-                    col.push_back(AP.col[k]);
-                    val.push_back(v);
-                }
-            }
+            for (int k = AP.ptr[i]; k < AP.ptr[i + 1]; k++) o.p.add(AP.col[k], acc[AP.col[k]] - d[i] * AP.val[k]);
             for (int k = h.P.ptr[i]; k < h.P.ptr[i + 1]; k++) acc[h.P.col[k]] = 0.0;
-            const int anchor = col.empty() ? 0 : col[0];
-            o.rows_u[i].y = tp.row(col.data(), val.data(), nullptr, (int)col.size(), anchor);
-            o.rows_u[i].z = (uint32_t)anchor;
+            o.p.end_row();
         }
-        o.off_p = std::move(tp.off);
-        o.v_p = std::move(tp.v);
         // Rt = R - R A w D^-1
         hf::HostCSR RA = hf::csr_multiply(h.R, h.A);
-        const int nn = h.R.n;
-        o.rows_r.resize(nn);
-        for (int i = 0; i < nn; i++) {
+        for (int i = 0; i < h.R.n; i++) {
             for (int k = h.R.ptr[i]; k < h.R.ptr[i + 1]; k++) acc[h.R.col[k]] = h.R.val[k];
-            col.clear();
-            val.clear();
-            for (int k = RA.ptr[i]; k < RA.ptr[i + 1]; k++) {
-                const double v = acc[RA.col[k]] - RA.val[k] * d[RA.col[k]];
-                if (v != 0.0) {
-                    col.push_back(RA.col[k]);
-                    val.push_back(v);
-                }
-            }
+            for (int k = RA.ptr[i]; k < RA.ptr[i + 1]; k++) o.r.add(RA.col[k], acc[RA.col[k]] - RA.val[k] * d[RA.col[k]]);
             for (int k = h.R.ptr[i]; k < h.R.ptr[i + 1]; k++) acc[h.R.col[k]] = 0.0;
-            const int anchor = col.empty() ? 0 : col[0];
-            o.rows_r[i] = make_uint2(tr.row(col.data(), val.data(), nullptr, (int)col.size(), anchor), (uint32_t)anchor);
+            o.r.end_row();
         }
-        o.off_r = std::move(tr.off);
-        o.v_r = std::move(tr.v);
-        if (!tp.ok || !tr.ok) return S;
+    }
+    // Rows of the coarse levels in the order of the fine rows they stand for:
+    // aggregation numbers leftover rows (the pinned cell, corners) last, and a
+    // rank that owned them would hold most of every vector.
+    std::vector<int> fine_pos;
+    for (int l = 0; l < S.clev; l++) {
+        const hf::HostLevel &h = H[l];
+        const int nn = h.R.n;
+        std::vector<std::pair<double, int>> key(nn);
+        for (int i = 0; i < nn; i++) {
+            double sum = 0.0;
+            const int a = h.R.ptr[i], e = h.R.ptr[i + 1];
+            for (int k = a; k < e; k++) sum += l == 0 ? h.R.col[k] : fine_pos[h.R.col[k]];
+            key[i] = {e > a ? sum / (e - a) : 0.0, i};
+        }
+        std::sort(key.begin(), key.end());
+        std::vector<int> pos(nn);
+        for (int i = 0; i < nn; i++) pos[key[i].second] = i;
+        HostSolve::Level &o = S.L[l];
+        o.r = permuted(o.r, pos, fine_pos);
+        o.p = permuted(o.p, fine_pos, pos);
+        if (l + 1 < S.clev) S.L[l + 1].m = permuted(S.L[l + 1].m, pos, pos);
+        else S.cpos = pos;
+        fine_pos = std::move(pos);
     }
     ranges(S);
     S.ok = true;
     return S;
+}
+
+// the instance's tables and its shared-memory layout
+template <typename T>
+struct Packed {
+    SInst<T> inst;
+    std::vector<SRank> ranks;
+    std::vector<char> tables, rank_tables;
+    size_t smem = 0;
+    bool ok = false;
+};
+
+template <typename T>
+Packed<T> pack(const HostSolve &S, const std::vector<double> &inverse, bool mixed)
+{
+    Packed<T> K;
+    SInst<T> &o = K.inst;
+    memset(&o, 0, sizeof o);
+    const int C = S.cluster, nt = S.threads;
+    o.n = S.L[0].n;
+    o.clev = S.clev;
+    o.nc = S.nc;
+    for (int l = 0; l < (int)S.L.size(); l++) o.lvl[l] = S.L[l].n;
+    size_t at = 0;
+    auto round = [](size_t b) { return (b + 15) & ~size_t(15); };
+    auto take = [&](size_t bytes) -> uint32_t {
+        if (at + round(bytes) > (size_t)kSolveSmem) return kSolveGlobal;
+        const uint32_t r = (uint32_t)at;
+        at += round(bytes);
+        return r;
+    };
+    // the vectors that are gathered from or exchanged always live in shared
+    // memory, at element indices of 16 bits
+    o.cvec = take(sizeof(T) * 2 * S.nc);
+    o.vr = take(sizeof(T) * S.held[0]);
+    o.vz = take(sizeof(T) * S.held[1]);
+    for (int l = 1; l < S.clev; l++) {
+        o.vb[l] = take(sizeof(T) * S.held[2 * l]);
+        o.vo[l] = take(sizeof(T) * S.held[2 * l + 1]);
+        if (o.vb[l] == kSolveGlobal || o.vo[l] == kSolveGlobal) return K;
+    }
+    if (o.cvec == kSolveGlobal || o.vr == kSolveGlobal || o.vz == kSolveGlobal || at / sizeof(T) > 0xffff) return K;
+    o.vq = take(sizeof(T) * S.held[0]);
+    if (o.vq == kSolveGlobal) return K;
+    const int own = (o.n + C - 1) / C;
+    auto blob = [&](std::vector<char> &to, const void *data, size_t bytes) {
+        const uint32_t g = (uint32_t)to.size();
+        to.insert(to.end(), (const char *)data, (const char *)data + bytes);
+        to.resize(round(to.size()), 0);
+        return g;
+    };
+    auto part = [&](const void *data, size_t bytes) {
+        STab t;
+        t.bytes = (uint32_t)round(bytes);
+        t.s = take(bytes);
+        t.g = blob(K.tables, data, bytes);
+        return t;
+    };
+    auto vals = [](const std::vector<double> &v) { return std::vector<T>(v.begin(), v.end()); };
+    auto ents = [&](const std::vector<double> &v) {
+        std::vector<SEnt<T>> e(v.size());
+        memset((void *)e.data(), 0, e.size() * sizeof(SEnt<T>));
+        for (size_t k = 0; k < e.size(); k++) {
+            e[k].off = S.off[k] * (int)sizeof(T);
+            e[k].v = (T)v[k];
+        }
+        return part(e.data(), e.size() * sizeof(SEnt<T>));
+    };
+    K.ranks.resize(C);
+    memset((void *)K.ranks.data(), 0, C * sizeof(SRank));
+    o.a = ents(S.va);
+    o.m = ents(S.vm);
+    if (o.a.s == kSolveGlobal || o.m.s == kSolveGlobal) return K;
+    // element index of row i of a vector in rank k's shared memory
+    auto elem = [&](uint32_t off, int vec, int k, int i) {
+        return (uint32_t)(off / sizeof(T)) + (uint32_t)(i - S.rng[(size_t)vec * C + k].x);
+    };
+    // one operator's rows of every rank in slices; f adds row i's entries
+    using Row = std::vector<std::pair<uint16_t, T>>;
+    auto slices = [&](int rows, int lg_max, auto f, SOp (SRank::*arr)[kMaxLevels], int l) {
+        size_t most = 0;
+        std::vector<std::vector<char>> data(C);
+        double entries = 0;
+        std::vector<std::vector<Row>> R(C);
+        for (int k = 0; k < C; k++) {
+            int a, h;
+            rank_rows(k, C, rows, a, h);
+            R[k].resize(h - a);
+            for (int i = a; i < h; i++) {
+                f(k, i, R[k][i - a]);
+                entries += (double)R[k][i - a].size();
+            }
+        }
+        const int m = (rows + C - 1) / C;
+        const double avg = entries / std::max(1, rows);
+        // threads per row: while the block has idle threads and a thread keeps
+        // a few entries
+        int lg = 0;
+        while (lg < lg_max && ((long)m << (lg + 1)) <= nt && avg > 3.0 * (1 << (lg + 1))) lg++;
+        for (int k = 0; k < C; k++) {
+            int a, h;
+            rank_rows(k, C, rows, a, h);
+            SOp &op = (K.ranks[k].*arr)[l];
+            op.row0 = a;
+            op.rows = h - a;
+            op.lg = lg;
+            const int per = 32 >> lg, lanes = 1 << lg;
+            op.nsl = (op.rows + per - 1) / per;
+            std::vector<uint32_t> ptr(1, 0);
+            std::vector<T> val;
+            std::vector<uint16_t> idx;
+            for (int s = 0; s < op.nsl; s++) {
+                int turns = 0;
+                for (int j = 0; j < per && s * per + j < op.rows; j++)
+                    turns = std::max(turns, ((int)R[k][s * per + j].size() + lanes - 1) / lanes);
+                const size_t b = val.size();
+                val.resize(b + (size_t)turns * 32, T(0));
+                idx.resize(b + (size_t)turns * 32, 0);
+                for (int j = 0; j < per && s * per + j < op.rows; j++) {
+                    const Row &row = R[k][s * per + j];
+                    for (size_t q = 0; q < row.size(); q++) {
+                        const size_t w = b + (q / lanes) * 32 + j * lanes + q % lanes;
+                        idx[w] = row[q].first;
+                        val[w] = row[q].second;
+                    }
+                }
+                ptr.push_back((uint32_t)(val.size() / 32));
+            }
+            std::vector<char> &c = data[k];
+            auto push = [&](const void *p, size_t bytes) {
+                const uint32_t w = (uint32_t)c.size();
+                c.insert(c.end(), (const char *)p, (const char *)p + bytes);
+                c.resize(round(c.size()), 0);
+                return w;
+            };
+            push(ptr.data(), ptr.size() * 4);
+            op.val = push(val.data(), val.size() * sizeof(T));
+            op.idx = push(idx.data(), idx.size() * 2);
+            most = std::max(most, c.size());
+        }
+        const uint32_t s = take(most);
+        for (int k = 0; k < C; k++) {
+            SOp &op = (K.ranks[k].*arr)[l];
+            op.t.s = s;
+            op.t.bytes = (uint32_t)data[k].size();
+            op.t.g = blob(K.rank_tables, data[k].data(), data[k].size());
+        }
+    };
+    auto add = [](Row &row, const Csr &A, int i, auto index) {
+        for (int q = A.ptr[i]; q < A.ptr[i + 1]; q++) row.emplace_back((uint16_t)index(A.col[q]), (T)A.val[q]);
+    };
+    // level l's out (the coarsest level's: co)
+    auto out_elem = [&](int l, int k, int i) {
+        return l == S.clev ? (uint32_t)(o.cvec / sizeof(T)) + S.nc + i : elem(o.vo[l], 2 * l + 1, k, i);
+    };
+    auto b_elem = [&](int l, int k, int i) { return l == 0 ? elem(o.vr, 0, k, i) : elem(o.vb[l], 2 * l, k, i); };
+    // the finest level's Pt and Rt as templates, where that form is the smaller
+    Tables tp, tr;
+    std::vector<uint32_t> dp(o.n, 0), dr;
+    int lg_r = 0;
+    if (S.clev > 0) {
+        const HostSolve::Level &L = S.L[0];
+        tp.pad = 2;
+        for (int i = 0; i < o.n; i++) {
+            const int a = L.p.ptr[i], len = L.p.ptr[i + 1] - a;
+            dp[i] = tp.row(L.p.col.data() + a, L.p.val.data() + a, nullptr, len, len ? L.p.col[a] : 0);
+        }
+        const int nr = L.r.rows(), m = (nr + C - 1) / C;
+        while (lg_r < 5 && ((long)m << (lg_r + 1)) <= nt && L.r.col.size() > 3.0 * nr * (1 << (lg_r + 1))) lg_r++;
+        tr.pad = 2 << lg_r;
+        dr.resize(nr);
+        for (int i = 0; i < nr; i++) {
+            const int a = L.r.ptr[i], len = L.r.ptr[i + 1] - a;
+            dr[i] = tr.row(L.r.col.data() + a, L.r.val.data() + a, nullptr, len, len ? L.r.col[a] : 0);
+        }
+        auto short_off = [](const Tables &t) {
+            for (int32_t v : t.off)
+                if (v < -32768 || v > 32767) return false;
+            return t.ok;
+        };
+        const size_t eb = sizeof(T) + 2;
+        // (with the row descriptors, and only where they fit beside the rest)
+        const size_t room = kSolveSmem - std::min<size_t>(kSolveSmem, at + sizeof(uint2) * own + sizeof(uint2) * m + 64);
+        const size_t bp = tp.off.size() * eb, br = tr.off.size() * eb;
+        o.tpl_r = short_off(tr) && br + 64 < room && br < L.r.col.size() / C * eb / 2;
+        o.tpl_p = short_off(tp) && bp + 64 < room - (o.tpl_r ? br : 0) && bp < L.p.col.size() / C * eb;
+    }
+    o.lg_r = lg_r;
+    {
+        // the finest level's own rows
+        std::vector<std::vector<uint2>> d(C);
+        for (int k = 0; k < C; k++) {
+            int lo, hi;
+            rank_rows(k, C, o.n, lo, hi);
+            for (int i = lo; i < hi; i++) {
+                uint32_t anchor = 0;
+                if (S.clev > 0 && S.L[0].p.ptr[i + 1] > S.L[0].p.ptr[i]) anchor = out_elem(1, k, S.L[0].p.col[S.L[0].p.ptr[i]]);
+                d[k].push_back(make_uint2(o.tpl_p ? dp[i] : 0u, anchor << 16 | S.tpl[i]));
+            }
+        }
+        const uint32_t s = take(sizeof(uint2) * own);
+        if (s == kSolveGlobal) return K;
+        for (int k = 0; k < C; k++) {
+            STab &t = K.ranks[k].desc0;
+            t.s = s;
+            t.bytes = (uint32_t)round(sizeof(uint2) * d[k].size());
+            t.g = blob(K.rank_tables, d[k].data(), sizeof(uint2) * d[k].size());
+        }
+    }
+    auto tables16 = [&](const Tables &t, STab &v, STab &f) {
+        std::vector<T> tv = vals(t.v);
+        std::vector<int16_t> to(t.off.begin(), t.off.end());
+        v = part(tv.data(), tv.size() * sizeof(T));
+        f = part(to.data(), to.size() * 2);
+    };
+    if (S.clev > 0) {
+        const HostSolve::Level &L = S.L[0];
+        if (o.tpl_r) {
+            tables16(tr, o.trv, o.tro);
+            std::vector<std::vector<uint2>> d(C);
+            size_t most = 0;
+            for (int k = 0; k < C; k++) {
+                int a, h;
+                rank_rows(k, C, L.r.rows(), a, h);
+                for (int i = a; i < h; i++)
+                    d[k].push_back(make_uint2(dr[i], L.r.ptr[i + 1] > L.r.ptr[i] ? b_elem(0, k, L.r.col[L.r.ptr[i]]) : 0u));
+                most = std::max(most, d[k].size());
+            }
+            const uint32_t s = take(sizeof(uint2) * most);
+            if (s == kSolveGlobal || o.trv.s == kSolveGlobal || o.tro.s == kSolveGlobal) return K;
+            for (int k = 0; k < C; k++) {
+                STab &t = K.ranks[k].desc_r;
+                t.s = s;
+                t.bytes = (uint32_t)round(sizeof(uint2) * d[k].size());
+                t.g = blob(K.rank_tables, d[k].data(), sizeof(uint2) * d[k].size());
+            }
+        }
+        if (o.tpl_p) {
+            tables16(tp, o.tpv, o.tpo);
+            if (o.tpv.s == kSolveGlobal || o.tpo.s == kSolveGlobal) return K;
+        }
+    }
+    for (int l = S.clev - 1; l > 0; l--) {
+        const HostSolve::Level &L = S.L[l];
+        slices(L.n, 5, [&](int k, int i, Row &row) {
+            add(row, L.m, i, [&](int c) { return b_elem(l, k, c); });
+            add(row, L.p, i, [&](int c) { return out_elem(l + 1, k, c); });
+        }, &SRank::up, l);
+        slices(L.r.rows(), 5, [&](int k, int i, Row &row) { add(row, L.r, i, [&](int c) { return b_elem(l, k, c); }); },
+               &SRank::down, l);
+    }
+    {
+        std::vector<T> d(inverse.size());
+        for (int i = 0; i < S.nc; i++)
+            for (int j = 0; j < S.nc; j++)
+                d[(size_t)(S.cpos.empty() ? i : S.cpos[i]) * S.nc + (S.cpos.empty() ? j : S.cpos[j])] =
+                    (T)inverse[(size_t)i * S.nc + j];
+        o.inv = part(d.data(), d.size() * sizeof(T));
+    }
+    if (S.clev > 0) {
+        const HostSolve::Level &L = S.L[0];
+        if (!o.tpl_r)
+            slices(L.r.rows(), 5, [&](int k, int i, Row &row) { add(row, L.r, i, [&](int c) { return b_elem(0, k, c); }); },
+                   &SRank::down, 0);
+        if (!o.tpl_p)
+            slices(L.n, 0, [&](int k, int i, Row &row) { add(row, L.p, i, [&](int c) { return out_elem(1, k, c); }); },
+                   &SRank::up, 0);
+    }
+    o.vp = take(sizeof(T) * own);
+    o.vx = take((mixed ? sizeof(T) : sizeof(double)) * own);
+    if (mixed) {
+        std::vector<SEnt<double>> e(S.off.size());
+        for (size_t q = 0; q < e.size(); q++) e[q] = SEnt<double>{S.va[q], S.off[q], 0};
+        o.a64.g = blob(K.tables, e.data(), e.size() * sizeof(SEnt<double>));
+        o.a64.s = kSolveGlobal;
+    }
+    K.smem = at;
+    K.ok = K.tables.size() < 0xffffffffu && K.rank_tables.size() < 0xffffffffu;
+    return K;
 }
 
 }  // namespace solve

@@ -1,0 +1,48 @@
+"""The one-launch Poisson solve (csrc/hf_solve.cuh) at the sizes where its
+partition changes: a finest level that is the coarsest (one dense solve), one
+CTA, the row counts around each cluster size, ragged last ranks, 3D rows, and
+batches whose instances take different cluster sizes; against the same steps in
+64-bit torch (perf/cases.py, exact()).
+
+Tolerances: the plain form at Poisson rtol 1e-13 is held to the suite's plain
+bar (1e-10 relative L2), the mixed form at the default rtol to the mixed bar
+(1e-6: FP32 stencil weights and convection)."""
+import importlib.util
+import os
+
+import numpy as np
+import pytest
+
+from higflow_b200 import engine
+from higflow_b200 import program as hp
+
+pytestmark = pytest.mark.gpu
+
+_spec = importlib.util.spec_from_file_location(
+    "perf_cases", os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "perf", "cases.py"))
+cases = importlib.util.module_from_spec(_spec)
+_spec.loader.exec_module(cases)
+
+SIZES = ["9x9", "12x11", "22x23", "23x23", "32x32", "33x31", "45x45", "46x46", "90x91", "91x91", "260x17", "129x128",
+         "9x9x9", "10x11x13", "17x16x17", "9,23,46,91", "32,91,10"]
+
+
+@pytest.mark.parametrize("precision", ["plain", "mixed"])
+@pytest.mark.parametrize("sides", SIZES)
+def test_steps_match_64_bit_steps(sides, precision):
+    flow = "giesekus" if sides in ("23x23", "91x91", "9,23,46,91", "10x11x13") else "newtonian"
+    case = dict(flow=flow, sides=sides, steps=3, precision=precision, scheme="explicit", per_step=False, limits="")
+    progs = cases._programs(case)
+    prog = progs[0] if len(progs) == 1 else hp.Program.concatenate(progs)
+    plain = precision == "plain"
+    opts = engine.options(precision=hp.PREC_FP64, rtol=1e-13, atol=1e-300) if plain else engine.options(precision=hp.PREC_MIXED)
+    c = engine.Case(prog, opts)
+    state = dict(case=c, fields=cases._inputs(case, 7)[1], steps=3, per_step=False, limits=None)
+    first = cases.run(state)
+    again = cases.run(state)
+    want = cases.exact(case, 7)
+    for k, w in want.items():
+        assert np.array_equal(first[k], again[k]), f"{k}: two runs differ"
+        err = np.linalg.norm(first[k] - w) / np.linalg.norm(w)
+        assert err < (1e-10 if plain else 1e-6), f"{k}: {err:.2e}"
+    c.close()
