@@ -203,6 +203,7 @@ struct Team {
 __device__ __forceinline__ void team_sync(const Team &t)
 {
     if (t.size > 1) {
+        __syncwarp();   // (.aligned: whole warps arrive)
         asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
         asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     } else {

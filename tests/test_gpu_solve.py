@@ -46,3 +46,20 @@ def test_steps_match_64_bit_steps(sides, precision):
         err = np.linalg.norm(first[k] - w) / np.linalg.norm(w)
         assert err < (1e-10 if plain else 1e-6), f"{k}: {err:.2e}"
     c.close()
+
+
+@pytest.mark.parametrize("sides", ["6x5", "16x17", "23x24", "32x33", "33x32", "65x64", "91x90", "128x129", "9x8x10"])
+def test_semi_implicit_steps_match_64_bit_steps(sides):
+    """The one-launch velocity systems (csrc/hf_bicg.cuh) around the sizes of
+    their 256-row blocks and ranks: systems of fewer rows than a block, one rank,
+    ragged last blocks, empty last ranks.  Two steps with both solves' residuals
+    at 1e-13: u to 1e-10, p (which follows u through div u* / dt, dt = 0.2 h^2)
+    to 1e-7."""
+    case = dict(flow="oldroyd", sides=sides, steps=2, precision="plain", scheme="semi_implicit", per_step=False, limits="")
+    prog = cases._programs(case)[0]
+    c = engine.Case(prog, engine.options(precision=hp.PREC_FP64, rtol=1e-13, atol=1e-300))
+    got = cases.run(dict(case=c, fields=cases._inputs(case, 7)[1], steps=2, per_step=False, limits=None))
+    for k, w in cases.exact(case, 7).items():
+        err = np.linalg.norm(got[k] - w) / np.linalg.norm(w)
+        assert err < (1e-7 if k == "p" else 1e-10), f"{k}: {err:.2e}"
+    c.close()
