@@ -1338,9 +1338,8 @@ __global__ void __launch_bounds__(kBlock) k_slv_init(DevMat M, BiVec V, double r
 // final velocity and pressure
 // ---------------------------------------------------------------------------
 template <int D>
-__global__ void __launch_bounds__(kBlock) k_final(DevProg P, DevFields F)
+__device__ __forceinline__ void final_element(const DevProg &P, const DevFields &F, int e)
 {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e < P.off[D]) {
         int d = 0;
 #pragma unroll
@@ -1365,6 +1364,26 @@ __global__ void __launch_bounds__(kBlock) k_final(DevProg P, DevFields F)
             (P.projtype_all >= 0 ? P.projtype_all : P.ipar[__ldg(P.cinst + c)].projtype) == HF_INCREMENTAL)
             F.p[c] = F.p[c] + F.dp[c];
     }
+}
+
+// END: the grid's last block to finish then ends the step (step_end; it counts
+// the instances' step limits down, which every other block has read by then)
+template <int D, bool END>
+__global__ void __launch_bounds__(kBlock) k_final(DevProg P, DevFields F, PcgFine G)
+{
+    final_element<D>(P, F, blockIdx.x * blockDim.x + threadIdx.x);
+    if (!END) return;
+    __shared__ bool last;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        last = atomicAdd(&G.ctl->gcount, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    if (threadIdx.x == 0) G.ctl->gcount = 0;
+    step_end(G);
 }
 
 
@@ -2285,6 +2304,7 @@ int build_pcg(hf_case *C, const std::vector<int32_t> &mptr, const std::vector<in
     const size_t o_r = ar.zeros<double>(n), o_z = ar.zeros<double>(n), o_q = ar.zeros<double>(n);
     const size_t o_pa = ar.zeros<double>(n), o_pb = ar.zeros<double>(n), o_xprev = ar.zeros<double>(n),
                  o_xprev2 = ar.zeros<double>(n);
+    const size_t o_xw = fused ? ar.zeros<double>(n) : 0;
     const size_t o_part = ar.zeros<double>((size_t)LH[0].ablk.size() * 2);
     // mixed form: the inner solve's FP32 vectors
     size_t o_r32 = 0, o_z32 = 0, o_q32 = 0, o_e32 = 0, o_pa32 = 0, o_pb32 = 0;
@@ -2334,6 +2354,7 @@ int build_pcg(hf_case *C, const std::vector<int32_t> &mptr, const std::vector<in
     G.dp = C->F.dp;
     G.xprev = (double *)(base + o_xprev);
     G.xprev2 = (double *)(base + o_xprev2);
+    G.xw = fused ? (double *)(base + o_xw) : nullptr;
     G.cinst = C->P.cinst;
     G.r = (double *)(base + o_r);
     G.z = (double *)(base + o_z);
@@ -2507,18 +2528,21 @@ void enqueue_body(hf_case *C, cudaStream_t st, cudaGraphConditionalHandle cond, 
 // forked from st and joined to it (under capture: parallel branches)
 int enqueue_solve(hf_case *C, cudaStream_t st, int &kernels)
 {
-    auto launch = [&](const hf_case::SolveLaunch &L, cudaStream_t on) -> cudaError_t {
+    auto launch = [&](const hf_case::SolveLaunch &L, cudaStream_t on, bool early) -> cudaError_t {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)(L.count * L.cluster));
         cfg.blockDim = dim3((unsigned)L.threads);
         cfg.dynamicSmemBytes = L.smem;
         cfg.stream = on;
-        cudaLaunchAttribute attr[1];
+        cudaLaunchAttribute attr[2];
         attr[0].id = cudaLaunchAttributeClusterDimension;
         attr[0].val.clusterDim.x = (unsigned)L.cluster;
         attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        // programmatic launch behind k_pcg_init, which it follows on this stream
+        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[1].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr;
-        cfg.numAttrs = 1;
+        cfg.numAttrs = early ? 2 : 1;
         kernels++;
         const PcgFine &G = C->G;
         if (C->mixed)
@@ -2531,7 +2555,7 @@ int enqueue_solve(hf_case *C, cudaStream_t st, int &kernels)
     for (size_t k = 0; k < C->solves.size(); k++) {
         cudaStream_t on = k ? C->solve_streams[k - 1] : st;
         if (k) HF_CK(cudaStreamWaitEvent(on, C->solve_events[0], 0));
-        HF_CK(launch(C->solves[k], on));
+        HF_CK(launch(C->solves[k], on, C->solves.size() == 1 && !C->profile));
     }
     for (size_t k = 1; k < C->solves.size(); k++) {
         HF_CK(cudaEventRecord(C->solve_events[k], C->solve_streams[k - 1]));
@@ -2821,11 +2845,16 @@ void enqueue_pre(hf_case *C, DevFields &F, int &fixed)
     if (C->sie) C->sie_rc = sie_solves(C, C->sie_launches);   // eager steps only (no graph for this form)
     record(C, HF_PHASE_VELOCITY, 1);
     record(C, HF_PHASE_POISSON_INIT, 0);
-    k_pcg_extrapolate<<<blocks(C->P.ncell), kBlock, 0, st>>>(C->G);
-    k_pcg_init<D><<<C->G.nblk, kBlock, 0, st>>>(C->P, F, C->G);
+    if (C->fused) {
+        k_pcg_init<D, true><<<C->G.nblk, kBlock, 0, st>>>(C->P, F, C->G);
+    } else {
+        k_pcg_extrapolate<<<blocks(C->P.ncell), kBlock, 0, st>>>(C->G);
+        k_pcg_init<D, false><<<C->G.nblk, kBlock, 0, st>>>(C->P, F, C->G);
+        fixed++;
+    }
     record(C, HF_PHASE_POISSON_INIT, 1);
     record(C, HF_PHASE_POISSON_ITER, 0);
-    fixed += 3;
+    fixed++;
 }
 
 // ... and after them: per-instance totals, final velocity and pressure
@@ -2835,11 +2864,9 @@ void enqueue_post(hf_case *C, const DevFields &F, int &fixed)
     cudaStream_t st = C->stream;
     record(C, HF_PHASE_POISSON_ITER, 1);
     record(C, HF_PHASE_FINAL, 0);
-    // (k_final first: k_step_end counts the instances' step limits down)
-    k_final<D><<<blocks(C->nfacet_total + C->P.ncell), kBlock, 0, st>>>(C->P, F);
-    k_step_end<<<1, kBlock, 0, st>>>(C->G);
+    k_final<D, true><<<blocks(C->nfacet_total + C->P.ncell), kBlock, 0, st>>>(C->P, F, C->G);
     record(C, HF_PHASE_FINAL, 1);
-    fixed += 2;
+    fixed++;
 }
 
 // One step with eager launches: the host reads the loop control after each body.
@@ -3030,10 +3057,10 @@ int collect_phases(hf_case *C)
     if (ve) C->phase_launches[HF_PHASE_VE_CELL_MAIN] += 1;
     C->phase_launches[HF_PHASE_VELOCITY] += 1 + (C->P.vr.n ? 1 : 0) + (rk ? 1 : 0);
     if (C->P.vr.n) C->phase_launches[HF_PHASE_VELOCITY_ROWS] += 1;
-    C->phase_launches[HF_PHASE_POISSON_INIT] += 2;
+    C->phase_launches[HF_PHASE_POISSON_INIT] += C->fused ? 1 : 2;
     C->phase_launches[HF_PHASE_POISSON_ITER] += C->fused ? (int64_t)C->solves.size()
                                                          : (C->h_ctl->total_bodies - C->bodies0) * C->body_kernels;
-    C->phase_launches[HF_PHASE_FINAL] += 2;
+    C->phase_launches[HF_PHASE_FINAL] += 1;
     return HF_OK;
 }
 
@@ -3160,7 +3187,7 @@ int bicg_step(hf_case *C)
         rc = fail(C->h_scal->status == 1 ? HF_ERR_NOT_CONVERGED : C->h_scal->status, "Poisson BiCGStab failed");
     {
         PhaseTimer t(C, HF_PHASE_FINAL, launches);
-        k_final<D><<<blocks(C->nfacet_total + n), kBlock, 0, st>>>(C->P, C->F);
+        k_final<D, false><<<blocks(C->nfacet_total + n), kBlock, 0, st>>>(C->P, C->F, C->G);
         launches++;
         t.stop(launches);
     }

@@ -208,6 +208,7 @@ struct PcgFine {
     const hf_params *ipar;
     double *p, *dp;           // unknown: dp (incremental projection) or p
     double *xprev, *xprev2;   // the unknown of the steps before (initial-guess extrapolation)
+    double *xw;               // the one-launch solve's initial guess (k_pcg_init), null otherwise
     const int32_t *cinst;     // cell -> instance
     double *r, *z, *q;
     double *partials;
@@ -409,11 +410,28 @@ __device__ __forceinline__ void csr_rows(const int32_t *__restrict__ ptr, const 
 
 }  // namespace pcg
 
+// Initial guess of the step's solve: extrapolation in time of the unknown from
+// the solutions of the steps before (x_n is the previous step's solution, the
+// reference's own initial guess, solver-petsc.c:386-399): quadratic,
+// x0 = 3 x_n - 3 x_{n-1} + x_{n-2}, once two earlier solutions are known,
+// linear, 2 x_n - x_{n-1}, with one, x_n with none (Ctl::hist counts them;
+// a restart clears it).  The solution is the same to the solve's tolerance;
+// the extrapolated start is closer to it, so fewer iterations are needed.
+__device__ __forceinline__ double extrapolated(int hist, double xn, double x1, double x2)
+{
+    return hist >= 2 ? 3.0 * xn - 3.0 * x1 + x2 : hist == 1 ? 2.0 * xn - x1 : xn;
+}
+
 // divergence right-hand side of every instance and the first residual
-// (higflow_pressure, hig-flow-step.c:58-120, with the instance's own dt and pin)
-template <int D>
+// (higflow_pressure, hig-flow-step.c:58-120, with the instance's own dt and pin).
+// EXT: the initial guess too, formed at every entry's column from the unknown
+// and its history, and written to xw (the one-launch solve shifts the history:
+// a launch of its own for that, k_pcg_extrapolate, costs 6 us of a step)
+template <int D, bool EXT>
 __global__ void __launch_bounds__(kBlock) k_pcg_init(DevProg P, DevFields F, PcgFine G)
 {
+    // (the one-launch solve loads its tables meanwhile)
+    if (EXT) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     Blk B;
     pcg::load_blk(G.blk, G.S, B);   // a new solve: the done flags are reset here
     // a frozen instance keeps done (and fin) from its last solve
@@ -424,6 +442,8 @@ __global__ void __launch_bounds__(kBlock) k_pcg_init(DevProg P, DevFields F, Pcg
     const int pin = G.ipin[B.inst];
     const double pinv = pin >= 0 ? (incr ? P.ipinv[B.inst] - F.p[pin] : P.ipinv[B.inst]) : 0.0;
     const int n = P.ncell;
+    const int hist = EXT ? __ldg(&G.ctl->hist) : 0;
+    auto guess = [&](int j) { return EXT ? extrapolated(hist, x[j], G.xprev[j], G.xprev2[j]) : x[j]; };
     double part[2] = {0.0, 0.0};   // r.r, b.b
 #pragma unroll
     for (int q = 0; q < kRPT; q++) {
@@ -445,7 +465,8 @@ __global__ void __launch_bounds__(kBlock) k_pcg_init(DevProg P, DevFields F, Pcg
             borig = sumdudx / par.dt + G.brhs[cc];
         }
         const double bred = cc == pin ? pinv : -(borig - G.apin[cc] * pinv);
-        const double ax = trow(G.A, cc, [&](int j) { return x[j]; });
+        const double ax = trow(G.A, cc, guess);
+        if (EXT) G.xw[cc] = guess(cc);
         const double r = bred - ax;
         G.r[cc] = r;
         if (G.r32) {
@@ -841,13 +862,7 @@ __global__ void __launch_bounds__(kBlock) k_pcg_update(PcgFine G, const double *
     }
 }
 
-// Initial guess of the step's solve: extrapolation in time of the unknown from
-// the solutions of the steps before (x_n is the previous step's solution, the
-// reference's own initial guess, solver-petsc.c:386-399): quadratic,
-// x0 = 3 x_n - 3 x_{n-1} + x_{n-2}, once two earlier solutions are known,
-// linear, 2 x_n - x_{n-1}, with one, x_n with none (Ctl::hist counts them;
-// a restart clears it).  The solution is the same to the solve's tolerance;
-// the extrapolated start is closer to it, so fewer iterations are needed.
+// the level-synchronous loop's initial guess
 __global__ void __launch_bounds__(kBlock) k_pcg_extrapolate(PcgFine G)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -862,7 +877,7 @@ __global__ void __launch_bounds__(kBlock) k_pcg_extrapolate(PcgFine G)
     const int hist = __ldg(&G.ctl->hist);
     G.xprev2[i] = x1;
     G.xprev[i] = xn;
-    x[i] = hist >= 2 ? 3.0 * xn - 3.0 * x1 + x2 : hist == 1 ? 2.0 * xn - x1 : xn;
+    x[i] = extrapolated(hist, xn, x1, x2);
 }
 
 // restart the time history: the next extrapolation starts from the unknown's
@@ -876,8 +891,9 @@ __global__ void __launch_bounds__(kBlock) k_pcg_restart(PcgFine G)
     if (i == 0) G.ctl->hist = 0;
 }
 
-// end of a step: per-instance totals, the first failure, loop counters reset
-__global__ void __launch_bounds__(kBlock) k_step_end(PcgFine G)
+// end of a step: per-instance totals, the first failure, loop counters reset.
+// One block runs it, the last of the step's last kernel (k_final)
+__device__ __forceinline__ void step_end(const PcgFine &G)
 {
     Ctl *c = G.ctl;
     for (int i = threadIdx.x; i < G.ninst; i += kBlock) {

@@ -347,16 +347,6 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_solve(PcgFine G, SolveArgs
     if (tid < 2 * kSolveMaxCluster) (&slot[0][0])[tid] = 0.0;
     if (tid < kSolveWarps) warp_sums[tid] = 0.0;
     __syncthreads();
-    IScal &S = G.S[I.inst];
-    // (read by every CTA before its first team barrier, written after the last)
-    const bool idle = ((volatile const IScal &)S).done != 0;
-    if (idle) {
-        if (tid == 0 && t.rank == 0) S.fin = 1;
-        return;
-    }
-    const double tol2 = S.tol2;
-    double tol2in = S.tol2in, rr = S.rr;
-    int status = 0, iters = 0, iters_prev = 0, outer = 0;
     const int n = I.n, clev = I.clev;
     for (int k = tid; k < kSolveVecs * t.size; k += nt) rng[k / t.size][k % t.size] = I.rng[k];
     copy4(&Rk, I.ranks + t.rank, sizeof Rk);
@@ -422,8 +412,29 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_solve(PcgFine G, SolveArgs
     const uint32_t pb = I.vp - (uint32_t)lo * kT, xb = I.vx - (uint32_t)lo * (MIX ? kT : 8u);
     const int pt = G.projtype_all >= 0 ? G.projtype_all : G.ipar[I.inst].projtype;
     double *xg = (pt == HF_INCREMENTAL ? G.dp : G.p) + I.row0;
-    if (!MIX && xs)
-        for (int i = lo + tid; i < hi; i += nt) at<double>(xb + 8u * i) = xg[i];
+    // Everything so far was the case's constant data, and overlaps k_pcg_init;
+    // from here on its results are read
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (G.ilim && G.ilim[I.inst] == 0) return;   // frozen: nothing changes
+    IScal &S = G.S[I.inst];
+    // (read by every CTA before its first team barrier, written after the last)
+    const bool idle = ((volatile const IScal &)S).done != 0;
+    // the unknown's history, and its initial guess in place
+    for (int i = lo + tid; i < hi; i += nt) {
+        const int j = I.row0 + i;
+        const double w = G.xw[j];
+        G.xprev2[j] = G.xprev[j];
+        G.xprev[j] = xg[i];
+        if (!MIX && xs && !idle) at<double>(xb + 8u * i) = w;
+        else xg[i] = w;
+    }
+    if (idle) {
+        if (tid == 0 && t.rank == 0) S.fin = 1;
+        return;
+    }
+    const double tol2 = S.tol2;
+    double tol2in = S.tol2in, rr = S.rr;
+    int status = 0, iters = 0, iters_prev = 0, outer = 0;
     for (int i = xlo + tid; i < xhi; i += nt) at<T>(r.row(i)) = A.r[I.row0 + i];
     const uint32_t tabA = I.a.s, tabM = I.m.s, desc = Rk.desc0.s - 8u * (uint32_t)lo;
     const int kk = K > 0 ? K : kf;
