@@ -1485,6 +1485,7 @@ struct hf_case {
     // one launch per cluster size runs the whole solve of its instances
     // (hf_solve.cuh) in place of the loop of level-synchronous kernels
     bool fused = false;
+    bool folded = false;            // otherwise: the loop runs the folded V-cycle (k_vf_*)
     struct SolveLaunch {
         int first, count, cluster, fine, threads;
         size_t smem;
@@ -1900,7 +1901,7 @@ VLev<T> make_level(char *base, const LevelOff &o, const LevelHost &h, const TRow
     VLev<T> v{};
     v.n = h.n;
     if (fine) {
-        v.At = At;
+        v.At = At;   // (the folded V-cycle's Mt below, where it is placed)
     } else {
         v.Ap = (const int32_t *)(base + o.Ap);
         v.Ac = (const int32_t *)(base + o.Ac);
@@ -2089,6 +2090,40 @@ int build_pcg(hf_case *C, const std::vector<int32_t> &mptr, const std::vector<in
         fused = all;
     }
     C->fused = fused;
+    // A case beyond that runs the level-synchronous loop on the folded
+    // operators; the semi-implicit form and BiCGStab's preconditioner keep the
+    // separate smoothing sweeps (their results follow its last bits)
+    bool folded = C->use_cg && amg && !C->sie && !fused;
+    struct Folded {
+        solve::Csr m, p, r;
+    };
+    std::vector<std::vector<Folded>> FO(folded ? ni : 0);
+    for (int i = 0; i < (int)FO.size(); i++) {
+        FO[i].resize(clev[i] + 1);
+        std::vector<std::thread> th;
+        for (int l = 0; l <= clev[i]; l++)
+            th.emplace_back([&FO, &IH, i, l]() { solve::fold(IH[i].H[l], &FO[i][l].m, FO[i][l].p, FO[i][l].r); });
+        for (auto &t : th) t.join();
+    }
+    TemplateForm fold_m0;   // the finest Mt: its rows are as many as A's, whose templates exist
+    if (folded) {
+        std::vector<int32_t> fp(1, 0), fc;
+        std::vector<double> fv;
+        for (int i = 0; i < ni; i++) {
+            const solve::Csr &m = FO[i][0].m;
+            for (int r = 0; r < m.rows(); r++) {
+                for (int k = m.ptr[r]; k < m.ptr[r + 1]; k++) {
+                    fc.push_back(m.col[k] + C->coff[i]);
+                    fv.push_back(m.val[k]);
+                }
+                fp.push_back((int32_t)fc.size());
+            }
+        }
+        fold_m0 = make_templates(fp, fc, fv, true);
+        folded = fold_m0.ok;
+    }
+    C->folded = folded;
+    const int tail_rows = folded ? kFoldTailRows : kTailRows;
     int nlev = 1;
     for (int i = 0; i < ni; i++) nlev = std::max(nlev, clev[i] + 1);
     C->nlev = nlev;
@@ -2106,7 +2141,7 @@ int build_pcg(hf_case *C, const std::vector<int32_t> &mptr, const std::vector<in
     C->nreg = 0;
     for (int i = 0; i < ni && amg; i++) {
         int s = 0;
-        while (s < clev[i] && off[s][i + 1] - off[s][i] > kTailRows) s++;
+        while (s < clev[i] && off[s][i + 1] - off[s][i] > tail_rows) s++;
         tail[i] = s;
         C->nreg = std::max(C->nreg, s);
     }
@@ -2145,16 +2180,18 @@ int build_pcg(hf_case *C, const std::vector<int32_t> &mptr, const std::vector<in
             for (int i = 0; i < ni; i++) {
                 if (clev[i] < l) continue;
                 const hf::HostLevel &hl = IH[i].H[l];
+                const std::vector<int> &ap = folded ? FO[i][l].m.ptr : hl.A.ptr, &ac = folded ? FO[i][l].m.col : hl.A.col;
+                const std::vector<double> &av = folded ? FO[i][l].m.val : hl.A.val;
                 for (int r = 0; r < hl.A.n; r++) {
-                    for (int k = hl.A.ptr[r]; k < hl.A.ptr[r + 1]; k++) {
-                        h.Ac.push_back(hl.A.col[k] + off[l][i]);
-                        h.Av.push_back(hl.A.val[k]);
+                    for (int k = ap[r]; k < ap[r + 1]; k++) {
+                        h.Ac.push_back(ac[k] + off[l][i]);
+                        h.Av.push_back(av[k]);
                     }
                     h.Ap.push_back((int32_t)h.Ac.size());
                 }
                 for (double d : hl.dinv) h.dinv.push_back(hl.omega * d);
+                C->lnnz_a[l] += (int64_t)hl.A.col.size();
             }
-            C->lnnz_a[l] = (int64_t)h.Ac.size();
         }
         if (l + 1 < nlev) {
             // P: rows of this level -> next level; R: rows of the next level -> this level
@@ -2168,23 +2205,26 @@ int build_pcg(hf_case *C, const std::vector<int32_t> &mptr, const std::vector<in
                     continue;
                 }
                 const hf::HostLevel &hl = IH[i].H[l];
-                for (int r = 0; r < hl.P.n; r++) {
-                    for (int k = hl.P.ptr[r]; k < hl.P.ptr[r + 1]; k++) {
-                        h.Pc.push_back(hl.P.col[k] + off[l + 1][i]);
-                        h.Pv.push_back(hl.P.val[k]);
+                auto append = [](const std::vector<int> &p, const std::vector<int> &c, const std::vector<double> &v, int o,
+                               std::vector<int32_t> &hp, std::vector<int32_t> &hc, std::vector<double> &hv) {
+                    for (size_t r = 0; r + 1 < p.size(); r++) {
+                        for (int k = p[r]; k < p[r + 1]; k++) {
+                            hc.push_back(c[k] + o);
+                            hv.push_back(v[k]);
+                        }
+                        hp.push_back((int32_t)hc.size());
                     }
-                    h.Pp.push_back((int32_t)h.Pc.size());
+                };
+                if (folded) {
+                    append(FO[i][l].p.ptr, FO[i][l].p.col, FO[i][l].p.val, off[l + 1][i], h.Pp, h.Pc, h.Pv);
+                    append(FO[i][l].r.ptr, FO[i][l].r.col, FO[i][l].r.val, off[l][i], h.Rp, h.Rc, h.Rv);
+                } else {
+                    append(hl.P.ptr, hl.P.col, hl.P.val, off[l + 1][i], h.Pp, h.Pc, h.Pv);
+                    append(hl.R.ptr, hl.R.col, hl.R.val, off[l][i], h.Rp, h.Rc, h.Rv);
                 }
-                for (int r = 0; r < hl.R.n; r++) {
-                    for (int k = hl.R.ptr[r]; k < hl.R.ptr[r + 1]; k++) {
-                        h.Rc.push_back(hl.R.col[k] + off[l][i]);
-                        h.Rv.push_back(hl.R.val[k]);
-                    }
-                    h.Rp.push_back((int32_t)h.Rc.size());
-                }
+                C->lnnz_p[l] += (int64_t)hl.P.col.size();
+                C->lnnz_r[l] += (int64_t)hl.R.col.size();
             }
-            C->lnnz_p[l] = (int64_t)h.Pc.size();
-            C->lnnz_r[l] = (int64_t)h.Rc.size();
         }
         h.sblk = block_table(off, tail, l, true);
         h.ablk = block_table(off, tail, l, false);
@@ -2277,6 +2317,7 @@ int build_pcg(hf_case *C, const std::vector<int32_t> &mptr, const std::vector<in
     }
     // template forms of the operators and transfers the level-synchronous
     // kernels read (levels above the last tail start); the tails keep CSR
+    if (folded) LH[0].At = std::move(fold_m0);
     if (amg && !fused) {
         std::vector<std::thread> th;
         for (int l = 0; l < C->nreg && l + 1 < nlev; l++) {
@@ -2494,12 +2535,49 @@ void enqueue_vcycle(hf_case *C, cudaStream_t st, const VLev<T> *L, const VLev<T>
     kernels++;
 }
 
+// the folded V-cycle and z of it, r.z
+template <typename T>
+void enqueue_folded(hf_case *C, cudaStream_t st, const VLev<T> *L, const VLev<T> *H, const TailInst<T> *ti, const T *r, T *z,
+                    int &kernels)
+{
+    const IScal *S = C->G.S;
+    for (int l = 0; l < C->nreg; l++) {
+        if (!L[l + 1].nablk) continue;
+        launch_pdl(k_vf_down<T, T>, L[l + 1].nablk * kFoldSplit, kBlock, st, L[l], L[l + 1], l == 0 ? r : (const T *)L[l].b, S);
+        kernels++;
+    }
+    launch_pdl(k_vf_tail<T>, C->ninst, kFoldTailThreads, st, H, ti, r, S);
+    for (int l = C->nreg - 1; l > 0; l--) {
+        if (!L[l].nsblk) continue;
+        launch_pdl(k_vf_up<T>, L[l].nsblk, kBlock, st, L[l], (const T *)L[l + 1].out, S);
+        kernels++;
+    }
+    launch_pdl(k_vf_z<T>, C->G.nblk, kBlock, st, C->G, L[0], (const T *)(C->nlev > 1 ? L[1].out : nullptr), r, z);
+    kernels += 2;
+}
+
 // two CG iterations (the direction vectors alternate, so two keep the graph
 // static); cond == 0: eager launches, the body is only counted on the device
 void enqueue_body(hf_case *C, cudaStream_t st, cudaGraphConditionalHandle cond, int &kernels)
 {
     for (int it = 0; it < 2; it++) {
         const int set = it == 1 ? (cond ? 1 : 2) : 0;
+        if (C->folded && C->mixed) {
+            enqueue_folded<float>(C, st, C->L32, C->h32, C->t32, C->G.r32, C->G.z32, kernels);
+            float *po = it == 0 ? C->pa32 : C->pb32, *pn = it == 0 ? C->pb32 : C->pa32;
+            launch_pdl(k_pcg_dir32, C->G.nblk, kBlock, st, C->G, (const float *)po, pn);
+            launch_pdl(k_pcg_update32, C->G.nblk, kBlock, st, C->G, (const float *)pn, cond, set);
+            kernels += 2;
+            continue;
+        }
+        if (C->folded) {
+            enqueue_folded<double>(C, st, C->L64, C->h64, C->t64, C->G.r, C->G.z, kernels);
+            double *po = it == 0 ? C->pa : C->pb, *pn = it == 0 ? C->pb : C->pa;
+            launch_pdl(k_pcg_dir, C->G.nblk, kBlock, st, C->G, (const double *)po, pn);
+            launch_pdl(k_pcg_update, C->G.nblk, kBlock, st, C->G, (const double *)pn, cond, set);
+            kernels += 2;
+            continue;
+        }
         if (C->mixed) {
             // the inner FP32 iteration of the mixed form
             enqueue_vcycle<float, float>(C, st, C->L32, C->h32, C->t32, C->G.r32, kernels);

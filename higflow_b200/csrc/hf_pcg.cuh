@@ -299,12 +299,13 @@ __device__ bool inst_sum(double (&v)[NV], const Blk &B, double *partials, IScal 
 }
 
 // block descriptor and the instance's done flag, shared by the block
-__device__ __forceinline__ bool load_blk(const Blk *tab, const IScal *S, Blk &B)
+// (split: grid blocks per table entry)
+__device__ __forceinline__ bool load_blk(const Blk *tab, const IScal *S, Blk &B, int split = 1)
 {
     __shared__ Blk sb;
     __shared__ int sd;
     if (threadIdx.x == 0) {
-        sb = tab[blockIdx.x];
+        sb = tab[blockIdx.x / split];
         sd = ((volatile const IScal *)S)[sb.inst].done;
     }
     __syncthreads();
@@ -686,6 +687,215 @@ __global__ void __launch_bounds__(kBlock) k_vc_post(VLev<T> L, const IScal *S)
         else
             for (int k = L.Ap[i]; k < L.Ap[i + 1]; k++) s += L.Av[k] * L.x[L.Ac[k]];
         L.out[i] = L.x[i] + L.dinv[i] * (L.b[i] - s);
+    }
+}
+
+// ---------------------------------------------------------------------------
+// the folded V-cycle (hf_solve.cuh states its operators): one kernel per level
+// down, b_{l+1} = Rt b_l, and one up, out_l = Mt b_l + Pt out_{l+1}, in place of
+// smoothing, residual, transfer and smoothing again.  A level's At, Pt, Rt and
+// CSR arrays then hold Mt, Pt and Rt (the finest level's At: Mt).  What bounds
+// the loop on one large instance is the number of its launches: 9 instead of 20
+// per iteration on 512 x 512 cells
+// ---------------------------------------------------------------------------
+// b_next = Rt b on every row of the next level (src: the level's b, the CG
+// residual on the finest)
+constexpr int kFoldSplit = 4;
+template <typename T, typename R = T>
+__global__ void __launch_bounds__(kBlock) k_vf_down(VLev<T> L, VLev<T> Ln, const R *src, const IScal *S)
+{
+    pdl_wait();
+    Blk B;
+    if (pcg::load_blk(Ln.ablk, S, B, kFoldSplit)) return;
+    // four threads per row: the rows are long (27 entries in 2D, 70 in 3D) and
+    // few; kFoldSplit grid blocks share a block's rows, so that a thread sums one
+    // row of a level of one row per thread
+    const int g = threadIdx.x >> 2, lane = threadIdx.x & 3;
+    const int per = (B.cnt + kFoldSplit - 1) / kFoldSplit, lo = (int)(blockIdx.x % kFoldSplit) * per, hi = min(B.cnt, lo + per);
+    for (int b = lo; b < hi; b += kBlock / 4) {
+        const int t = b + g;
+        T s = T(0);
+        if (t < hi) {
+            const int i = B.row0 + t;
+            if (L.Rt.rb) {
+                const uint2 d = __ldg(L.Rt.rb + i);
+                const int k0 = (int)(d.x >> kTLenBits), e = k0 + (int)(d.x & ((1u << kTLenBits) - 1)), a = (int)d.y;
+#pragma unroll 8
+                for (int k = k0 + lane; k < e; k += 4) s += __ldg(L.Rt.tval + k) * T(src[a + __ldg(L.Rt.toff + k)]);
+            } else {
+                const int e = L.Rp[i + 1];
+#pragma unroll 8
+                for (int k = L.Rp[i] + lane; k < e; k += 4) s += __ldg(L.Rv + k) * T(src[__ldg(L.Rc + k)]);
+            }
+        }
+        s += __shfl_xor_sync(0xffffffffu, s, 1);
+        s += __shfl_xor_sync(0xffffffffu, s, 2);
+        if (t < hi && lane == 0) Ln.b[B.row0 + t] = s;
+    }
+}
+
+// Mt b + Pt e on a thread's rows
+template <typename T, typename Fn>
+__device__ __forceinline__ void folded_up(const VLev<T> &L, const pcg::RowSet &R, const T *e, T (&s)[kRPT], Fn b)
+{
+    // (a row's entries eight at a time: their loads are in flight together)
+#pragma unroll
+    for (int q = 0; q < kRPT; q++) {
+        s[q] = T(0);
+        if (q >= R.nrow) continue;
+        const int i = R.row[q];
+        T u = T(0), v = T(0);
+        if (L.At.rd) {
+            const uint32_t d = __ldg(L.At.rd + i);
+            const int k0 = (int)(d >> kTLenBits), n = (int)(d & ((1u << kTLenBits) - 1));
+#pragma unroll 8
+            for (int k = 0; k < n; k++) u += __ldg(L.At.tval + k0 + k) * b(i + __ldg(L.At.toff + k0 + k));
+        } else {
+            const int n = L.Ap[i + 1];
+#pragma unroll 8
+            for (int k = L.Ap[i]; k < n; k++) u += __ldg(L.Av + k) * b(__ldg(L.Ac + k));
+        }
+        if (L.Pt.rb) {
+            const uint2 d = __ldg(L.Pt.rb + i);
+            const int k0 = (int)(d.x >> kTLenBits), n = (int)(d.x & ((1u << kTLenBits) - 1)), a = (int)d.y;
+#pragma unroll 8
+            for (int k = 0; k < n; k++) v += __ldg(L.Pt.tval + k0 + k) * e[a + __ldg(L.Pt.toff + k0 + k)];
+        } else {
+            const int n = L.Pp[i + 1];
+#pragma unroll 8
+            for (int k = L.Pp[i]; k < n; k++) v += __ldg(L.Pv + k) * e[__ldg(L.Pc + k)];
+        }
+        s[q] = u + v;
+    }
+}
+
+// out = Mt b + Pt e on the smoothed rows of a coarse level
+template <typename T>
+__global__ void __launch_bounds__(kBlock) k_vf_up(VLev<T> L, const T *e, const IScal *S)
+{
+    pdl_wait();
+    Blk B;
+    if (pcg::load_blk(L.sblk, S, B)) return;
+    const pcg::RowSet R = pcg::rowset(B);
+    T s[kRPT];
+    folded_up(L, R, e, s, [&](int j) { return L.b[j]; });
+#pragma unroll
+    for (int q = 0; q < kRPT; q++)
+        if (q < R.nrow) L.out[R.row[q]] = s[q];
+}
+
+// z = Mt r + Pt e on the finest level (or the tail's output), r.z -> beta per
+// instance; r, z: the plain form's vectors or the mixed form's FP32 ones
+template <typename T>
+__global__ void __launch_bounds__(kBlock) k_vf_z(PcgFine G, VLev<T> L0, const T *e, const T *r, T *z)
+{
+    pdl_wait();
+    Blk B;
+    if (pcg::load_blk(G.blk, G.S, B)) return;
+    const bool tail0 = G.S[B.inst].tail0;
+    const pcg::RowSet R = pcg::rowset(B);
+    T s[kRPT];
+    if (!tail0) folded_up(L0, R, e, s, [&](int j) { return r[j]; });
+    double part[1] = {0.0};
+#pragma unroll
+    for (int q = 0; q < kRPT; q++) {
+        if (q >= R.nrow) break;
+        const int i = R.row[q];
+        const T zi = tail0 ? L0.out[i] : s[q];
+        z[i] = zi;
+        part[0] += (double)r[i] * (double)zi;
+    }
+    double tot[1];
+    if (pcg::inst_sum<1>(part, B, G.partials, G.S, tot) && threadIdx.x == 0) {
+        IScal &s = G.S[B.inst];
+        s.beta = s.iters == 0 ? 0.0 : tot[0] / s.rz;
+        s.rz = tot[0];
+        if (!isfinite(tot[0])) { s.status = HF_ERR_NAN; pcg::finish_instance(s, G.ctl); }
+    }
+}
+
+// the small levels of one instance, down and up, one CTA (as k_vc_tail): eight
+// threads per row down, one up
+constexpr int kFoldTailRows = 1024;
+constexpr int kFoldTailThreads = 1024;
+template <typename T>
+__global__ void __launch_bounds__(kFoldTailThreads) k_vf_tail(const VLev<T> *H, const TailInst<T> *TI, const T *r0, const IScal *S)
+{
+    pdl_wait();
+    __shared__ TailInst<T> ti;
+    __shared__ VLev<T> L, Ln;
+    __shared__ int done;
+    __shared__ T sb[kCoarseCap];
+    if (threadIdx.x == 0) {
+        ti = TI[blockIdx.x];
+        done = ((volatile const IScal *)S)[ti.inst].done;
+    }
+    __syncthreads();
+    if (done) return;
+    const int tid = threadIdx.x;
+    for (int l = ti.s; l < ti.clev; l++) {
+        if (tid == 0) {
+            L = H[l];
+            Ln = H[l + 1];
+        }
+        __syncthreads();
+        const T *b = l == 0 ? r0 : L.b;
+        const int a = ti.row0[l + 1], n = ti.nrow[l + 1], lane = tid & 7;
+        for (int t = tid >> 3; t - (tid >> 3) < n; t += kFoldTailThreads / 8) {
+            T s = T(0);
+            if (t < n)
+            {
+                const int e = L.Rp[a + t + 1];
+#pragma unroll 8
+                for (int k = L.Rp[a + t] + lane; k < e; k += 8) s += __ldg(L.Rv + k) * b[__ldg(L.Rc + k)];
+            }
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            if (t < n && lane == 0) Ln.b[a + t] = s;
+        }
+        __syncthreads();
+    }
+    // coarsest: out = inv b, one warp per row, lanes over the row
+    {
+        if (tid == 0) L = H[ti.clev];
+        __syncthreads();
+        const int a = ti.row0[ti.clev], cn = ti.nrow[ti.clev];
+        for (int i = tid; i < cn; i += kFoldTailThreads) sb[i] = ti.clev == 0 ? r0[a + i] : L.b[a + i];
+        __syncthreads();
+        const int lane = tid & 31, warp = tid >> 5;
+        for (int i = warp; i < cn; i += kFoldTailThreads / 32) {
+            const T *row = ti.inv + (size_t)i * cn;
+            T s = T(0);
+            for (int k = lane; k < cn; k += 32) s += row[k] * sb[k];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            if (lane == 0) L.out[a + i] = s;
+        }
+        __syncthreads();
+    }
+    for (int l = ti.clev - 1; l >= ti.s; l--) {
+        if (tid == 0) {
+            L = H[l];
+            Ln = H[l + 1];
+        }
+        __syncthreads();
+        const T *b = l == 0 ? r0 : L.b;
+        const int a = ti.row0[l], e = a + ti.nrow[l];
+        for (int i = a + tid; i < e; i += kFoldTailThreads) {
+            T s = T(0);
+            if (l == 0) {
+                s = trow(L.At, i, [&](int j) { return b[j]; });
+            } else {
+                const int n = L.Ap[i + 1];
+#pragma unroll 8
+                for (int k = L.Ap[i]; k < n; k++) s += __ldg(L.Av + k) * b[__ldg(L.Ac + k)];
+            }
+            const int n = L.Pp[i + 1];
+#pragma unroll 8
+            for (int k = L.Pp[i]; k < n; k++) s += __ldg(L.Pv + k) * Ln.out[__ldg(L.Pc + k)];
+            L.out[i] = s;
+        }
+        __syncthreads();
     }
 }
 

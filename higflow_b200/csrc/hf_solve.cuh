@@ -773,6 +773,40 @@ inline Csr permuted(const Csr &A, const std::vector<int> &rpos, const std::vecto
     return B;
 }
 
+// the folded operators of one level (m only where wanted)
+inline void fold(const hf::HostLevel &h, Csr *m, Csr &p, Csr &r)
+{
+    const int n = h.A.n;
+    std::vector<double> d(n);
+    for (int i = 0; i < n; i++) d[i] = h.omega * h.dinv[i];
+    if (m)
+        for (int i = 0; i < n; i++) {
+            for (int k = h.A.ptr[i]; k < h.A.ptr[i + 1]; k++) {
+                const int j = h.A.col[k];
+                m->add(j, (j == i ? 2.0 * d[i] : 0.0) - d[i] * h.A.val[k] * d[j]);
+            }
+            m->end_row();
+        }
+    if (h.P.ptr.empty()) return;   // the coarsest level
+    // Pt = P - w D^-1 A P
+    hf::HostCSR AP = hf::csr_multiply(h.A, h.P);
+    std::vector<double> acc(std::max(h.P.m, n), 0.0);
+    for (int i = 0; i < n; i++) {
+        for (int k = h.P.ptr[i]; k < h.P.ptr[i + 1]; k++) acc[h.P.col[k]] = h.P.val[k];
+        for (int k = AP.ptr[i]; k < AP.ptr[i + 1]; k++) p.add(AP.col[k], acc[AP.col[k]] - d[i] * AP.val[k]);
+        for (int k = h.P.ptr[i]; k < h.P.ptr[i + 1]; k++) acc[h.P.col[k]] = 0.0;
+        p.end_row();
+    }
+    // Rt = R - R A w D^-1
+    hf::HostCSR RA = hf::csr_multiply(h.R, h.A);
+    for (int i = 0; i < h.R.n; i++) {
+        for (int k = h.R.ptr[i]; k < h.R.ptr[i + 1]; k++) acc[h.R.col[k]] = h.R.val[k];
+        for (int k = RA.ptr[i]; k < RA.ptr[i + 1]; k++) r.add(RA.col[k], acc[RA.col[k]] - RA.val[k] * d[RA.col[k]]);
+        for (int k = h.R.ptr[i]; k < h.R.ptr[i + 1]; k++) acc[h.R.col[k]] = 0.0;
+        r.end_row();
+    }
+}
+
 struct HostSolve {
     bool ok = false;
     int clev = 0, nc = 0, cluster = 1, threads = 256, fine = 0;   // fine: entries of the finest operator's rows
@@ -892,8 +926,6 @@ inline HostSolve build(const std::vector<hf::HostLevel> &H, long total)
         HostSolve::Level &o = S.L[l];
         const int n = h.A.n;
         o.n = n;
-        std::vector<double> d(n);
-        for (int i = 0; i < n; i++) d[i] = h.omega * h.dinv[i];
         if (l == 0) {
             int most = 1;
             for (int i = 0; i < n; i++) most = std::max(most, h.A.ptr[i + 1] - h.A.ptr[i]);
@@ -903,10 +935,11 @@ inline HostSolve build(const std::vector<hf::HostLevel> &H, long total)
             std::vector<double> mv;
             for (int i = 0; i < n; i++) {
                 const int a = h.A.ptr[i], len = h.A.ptr[i + 1] - a;
+                const double di = h.omega * h.dinv[i];
                 mv.resize(len);
                 for (int k = 0; k < len; k++) {
                     const int j = h.A.col[a + k];
-                    mv[k] = (j == i ? 2.0 * d[i] : 0.0) - d[i] * h.A.val[a + k] * d[j];
+                    mv[k] = (j == i ? 2.0 * di : 0.0) - di * h.A.val[a + k] * (h.omega * h.dinv[j]);
                 }
                 S.tpl[i] = (tm.row(&h.A.col[a], mv.data(), &h.A.val[a], len, i) >> kSolveLenBits) / S.fine;
                 if (S.tpl[i] > 0xffffu) tm.ok = false;
@@ -915,33 +948,9 @@ inline HostSolve build(const std::vector<hf::HostLevel> &H, long total)
             S.off = std::move(tm.off);
             S.vm = std::move(tm.v);
             S.va = std::move(tm.v2);
-        } else {
-            for (int i = 0; i < n; i++) {
-                for (int k = h.A.ptr[i]; k < h.A.ptr[i + 1]; k++) {
-                    const int j = h.A.col[k];
-                    o.m.add(j, (j == i ? 2.0 * d[i] : 0.0) - d[i] * h.A.val[k] * d[j]);
-                }
-                o.m.end_row();
-            }
         }
         if (l >= S.clev) break;   // the finest level is the coarsest
-        // Pt = P - w D^-1 A P
-        hf::HostCSR AP = hf::csr_multiply(h.A, h.P);
-        std::vector<double> acc(std::max(h.P.m, n), 0.0);
-        for (int i = 0; i < n; i++) {
-            for (int k = h.P.ptr[i]; k < h.P.ptr[i + 1]; k++) acc[h.P.col[k]] = h.P.val[k];
-            for (int k = AP.ptr[i]; k < AP.ptr[i + 1]; k++) o.p.add(AP.col[k], acc[AP.col[k]] - d[i] * AP.val[k]);
-            for (int k = h.P.ptr[i]; k < h.P.ptr[i + 1]; k++) acc[h.P.col[k]] = 0.0;
-            o.p.end_row();
-        }
-        // Rt = R - R A w D^-1
-        hf::HostCSR RA = hf::csr_multiply(h.R, h.A);
-        for (int i = 0; i < h.R.n; i++) {
-            for (int k = h.R.ptr[i]; k < h.R.ptr[i + 1]; k++) acc[h.R.col[k]] = h.R.val[k];
-            for (int k = RA.ptr[i]; k < RA.ptr[i + 1]; k++) o.r.add(RA.col[k], acc[RA.col[k]] - RA.val[k] * d[RA.col[k]]);
-            for (int k = h.R.ptr[i]; k < h.R.ptr[i + 1]; k++) acc[h.R.col[k]] = 0.0;
-            o.r.end_row();
-        }
+        fold(h, l > 0 ? &o.m : nullptr, o.p, o.r);
     }
     // Rows of the coarse levels in the order of the fine rows they stand for:
     // aggregation numbers leftover rows (the pinned cell, corners) last, and a

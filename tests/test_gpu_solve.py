@@ -27,8 +27,12 @@ SIZES = ["9x9", "12x11", "22x23", "23x23", "32x32", "33x31", "45x45", "46x46", "
          "9x9x9", "10x11x13", "17x16x17", "9,23,46,91", "32,91,10"]
 
 
-@pytest.mark.parametrize("precision", ["plain", "mixed"])
-@pytest.mark.parametrize("sides", SIZES)
+# beyond one cluster: the level-synchronous loop on the folded operators, alone
+# and with instances that are all tail or all dense
+LARGE = [("300x299", "plain"), ("470x450", "mixed"), ("300,9,40", "plain"), ("460,33,9", "mixed")]
+
+
+@pytest.mark.parametrize("sides,precision", [(s, p) for p in ("plain", "mixed") for s in SIZES] + LARGE)
 def test_steps_match_64_bit_steps(sides, precision):
     flow = "giesekus" if sides in ("23x23", "91x91", "9,23,46,91", "10x11x13") else "newtonian"
     case = dict(flow=flow, sides=sides, steps=3, precision=precision, scheme="explicit", per_step=False, limits="")
