@@ -1433,6 +1433,50 @@ void keep_pool_memory(int dev)
 
 }  // namespace
 
+// Page-locked blocks for the cases of the process, any thread's: allocating and
+// freeing one waits for the device, so up to kPinKeep are kept for the next case.
+constexpr size_t kPinBytes = size_t(1) << 20;
+constexpr size_t kPinKeep = 16;
+constexpr size_t kStageMost = size_t(256) << 10;   // larger transfers go straight to the caller's memory
+struct PinnedPool {
+    std::mutex m;
+    std::vector<char *> blocks;
+    char *take()
+    {
+        {
+            std::lock_guard<std::mutex> g(m);
+            if (!blocks.empty()) {
+                char *b = blocks.back();
+                blocks.pop_back();
+                return b;
+            }
+        }
+        void *b = nullptr;
+        if (cudaHostAlloc(&b, kPinBytes, cudaHostAllocPortable) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        return (char *)b;
+    }
+    void give(char *b)
+    {
+        if (!b) return;
+        {
+            std::lock_guard<std::mutex> g(m);
+            if (blocks.size() < kPinKeep) {
+                blocks.push_back(b);
+                return;
+            }
+        }
+        cudaFreeHost(b);
+    }
+};
+PinnedPool &pinned_pool()
+{
+    static PinnedPool *p = new PinnedPool;   // outlives every case, also at exit
+    return *p;
+}
+
 struct hf_case {
     hf_options opt;
     hf_params par;
@@ -1499,8 +1543,16 @@ struct hf_case {
     std::vector<int64_t> lrows, lnnz_a, lnnz_p, lnnz_r;
     int body_kernels = 0;           // kernels of one loop body (two iterations)
     int fixed_kernels = 0;          // kernels of a step outside the loop
-    IScal *h_S = nullptr;           // pinned mirrors
+    IScal *h_S = nullptr;           // mirrors of the instance scalars and the loop control
     Ctl *h_ctl = nullptr;
+    // page-locked memory of the case (PinnedPool; null: none to be had): the
+    // mirrors, then a staging area for small transfers.  Staged copies in are
+    // queued on the case stream without waiting; the area starts over after a
+    // synchronisation.
+    char *pin = nullptr;
+    size_t stage0 = 0, stage_at = 0;
+    bool state_pinned = false;
+    bool state_fresh = false;       // the mirrors hold the state after the last step
     cudaStream_t body_stream = nullptr;
     cudaGraph_t graph[2] = {};
     cudaGraphExec_t exec[2] = {};
@@ -2477,8 +2529,19 @@ int build_pcg(hf_case *C, const std::vector<int32_t> &mptr, const std::vector<in
         }
         C->bytes += bytes;
     }
-    C->h_S = new IScal[ni]();
-    C->h_ctl = new Ctl();
+    // the mirrors: one page-locked stretch laid out as on the device, so that one
+    // copy fetches both
+    const size_t ctl_off = o_ctl - o_S, state = ctl_off + sizeof(Ctl);
+    if (C->pin && state <= kPinBytes / 2) {
+        memset(C->pin, 0, state);
+        C->h_S = (IScal *)C->pin;
+        C->h_ctl = (Ctl *)(C->pin + ctl_off);
+        C->state_pinned = true;
+        C->stage0 = C->stage_at = (state + 255) & ~size_t(255);
+    } else {
+        C->h_S = new IScal[ni]();
+        C->h_ctl = new Ctl();
+    }
     return HF_OK;
 }
 
@@ -3095,10 +3158,33 @@ int ensure_graphs(hf_case *C)
 // device -> host copies of the instance scalars and the loop control
 int pull_state(hf_case *C)
 {
-    HF_CK(cudaMemcpyAsync(C->h_S, C->G.S, sizeof(IScal) * C->ninst, cudaMemcpyDeviceToHost, C->stream));
-    HF_CK(cudaMemcpyAsync(C->h_ctl, C->G.ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, C->stream));
+    if (C->state_pinned) {
+        HF_CK(cudaMemcpyAsync(C->h_S, C->G.S, (char *)(C->h_ctl + 1) - (char *)C->h_S, cudaMemcpyDeviceToHost, C->stream));
+    } else {
+        HF_CK(cudaMemcpyAsync(C->h_S, C->G.S, sizeof(IScal) * C->ninst, cudaMemcpyDeviceToHost, C->stream));
+        HF_CK(cudaMemcpyAsync(C->h_ctl, C->G.ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, C->stream));
+    }
     HF_CK(cudaStreamSynchronize(C->stream));
+    C->stage_at = C->stage0;
+    C->state_fresh = true;
     return HF_OK;
+}
+
+// the mirrors as of the last step, fetched once per step
+int want_state(hf_case *C) { return C->state_fresh ? HF_OK : pull_state(C); }
+
+// a staging area of `bytes` for one transfer (null: too large, or none)
+char *stage(hf_case *C, size_t bytes)
+{
+    if (!C->pin || bytes > kStageMost) return nullptr;
+    bytes = (bytes + 255) & ~size_t(255);
+    if (C->stage_at + bytes > kPinBytes) {
+        if (cudaStreamSynchronize(C->stream) != cudaSuccess) return nullptr;
+        C->stage_at = C->stage0;
+    }
+    char *p = C->pin + C->stage_at;
+    C->stage_at += bytes;
+    return p;
 }
 
 // the first failed solve since the last check, as a status (then cleared)
@@ -3111,6 +3197,7 @@ int take_error(hf_case *C)
                       " at step " + std::to_string(c.err_step);
     HF_CK(cudaMemsetAsync(&C->G.ctl->err_status, 0, sizeof(int32_t), C->stream));
     HF_CK(cudaStreamSynchronize(C->stream));
+    C->h_ctl->err_status = 0;
     return fail(code, msg);
 }
 
@@ -3280,6 +3367,7 @@ int bicg_step(hf_case *C)
 
 int run_steps(hf_case *C, int nsteps, bool sync)
 {
+    if (nsteps > 0) C->state_fresh = false;
     if (!C->use_cg) {
         for (int s = 0; s < nsteps; s++) {
             int rc = C->D == 2 ? bicg_step<2>(C) : bicg_step<3>(C);
@@ -3493,6 +3581,7 @@ extern "C" int hf_case_create(const hf_program *pg, const hf_options *opt_in, hf
         cudaStreamCreateWithFlags(&C->body_stream, cudaStreamNonBlocking) != cudaSuccess)
         return cleanup(fail(HF_ERR_CUDA, "stream"));
     C->h_scal = new Scal();
+    C->pin = pinned_pool().take();
     keep_pool_memory(opt.device);
 
     DevProg &P = C->P;
@@ -3987,14 +4076,16 @@ extern "C" int hf_case_set_field(hf_case *C, int32_t field, int32_t comp, const 
     int64_t m = 0;
     double *p = field_ptr(C, field, comp, &m);
     if (!p || m != n) return fail(HF_ERR_INVALID, "field/component/size mismatch");
-    HF_CK(cudaMemcpyAsync(p, host, sizeof(double) * (size_t)n, cudaMemcpyHostToDevice, C->stream));
+    char *staged = stage(C, sizeof(double) * (size_t)n);
+    if (staged) memcpy(staged, host, sizeof(double) * (size_t)n);
+    HF_CK(cudaMemcpyAsync(p, staged ? (const void *)staged : host, sizeof(double) * (size_t)n, cudaMemcpyHostToDevice, C->stream));
     // a new value of the solve's unknown restarts its time history (the next
     // initial guess is the value itself, not an extrapolation)
     if (C->G.xprev && (field == HF_FIELD_DP || field == HF_FIELD_P)) {
         k_pcg_restart<<<blocks(C->P.ncell), kBlock, 0, C->stream>>>(C->G);
         HF_CK(cudaGetLastError());
     }
-    HF_CK(cudaStreamSynchronize(C->stream));
+    if (!staged) HF_CK(cudaStreamSynchronize(C->stream));   // the caller's memory is read until then
     return HF_OK;
 }
 
@@ -4004,8 +4095,11 @@ extern "C" int hf_case_get_field(hf_case *C, int32_t field, int32_t comp, double
     int64_t m = 0;
     double *p = field_ptr(C, field, comp, &m);
     if (!p || m != n) return fail(HF_ERR_INVALID, "field/component/size mismatch");
-    HF_CK(cudaMemcpyAsync(host, p, sizeof(double) * (size_t)n, cudaMemcpyDeviceToHost, C->stream));
+    char *staged = stage(C, sizeof(double) * (size_t)n);
+    HF_CK(cudaMemcpyAsync(staged ? (void *)staged : host, p, sizeof(double) * (size_t)n, cudaMemcpyDeviceToHost, C->stream));
     HF_CK(cudaStreamSynchronize(C->stream));
+    if (staged) memcpy(host, staged, sizeof(double) * (size_t)n);
+    C->stage_at = C->stage0;
     return HF_OK;
 }
 
@@ -4035,7 +4129,7 @@ extern "C" int hf_case_stats(hf_case *C, hf_stats *out)
 {
     if (!C || !out) return fail(HF_ERR_INVALID, "null argument");
     if (C->use_cg) {
-        int rc = pull_state(C);
+        int rc = want_state(C);
         if (rc) return rc;
         hf_stats &s = C->stats;
         s.last_iters = 0;
@@ -4074,7 +4168,7 @@ extern "C" int hf_case_instance_result(hf_case *C, int32_t inst, int32_t *iters,
         if (residual) *residual = C->stats.last_residual;
         return HF_OK;
     }
-    int rc = pull_state(C);
+    int rc = want_state(C);
     if (rc) return rc;
     const IScal &q = C->h_S[inst];
     if (iters) *iters = q.iters + q.iters_prev;
@@ -4138,11 +4232,13 @@ extern "C" int hf_case_set_timestep(hf_case *C, const double *dt, int32_t n)
         return fail(HF_ERR_UNSUPPORTED, "new time step with the semi-implicit velocity (its matrix holds dt)");
     }
     // (the parameters go to the device on every call, as the host's dt of
-    // each step; no step of this case is in flight past the synchronisation)
+    // each step, in the order of the case stream)
     for (int i = 0; i < n; i++) C->h_ipar[i].dt = dt[i];
-    HF_CK(cudaMemcpyAsync((void *)C->P.ipar, C->h_ipar.data(), sizeof(hf_params) * n, cudaMemcpyHostToDevice,
-                          C->stream));
-    HF_CK(cudaStreamSynchronize(C->stream));
+    char *staged = stage(C, sizeof(hf_params) * (size_t)n);
+    if (staged) memcpy(staged, C->h_ipar.data(), sizeof(hf_params) * (size_t)n);
+    HF_CK(cudaMemcpyAsync((void *)C->P.ipar, staged ? (const void *)staged : C->h_ipar.data(), sizeof(hf_params) * n,
+                          cudaMemcpyHostToDevice, C->stream));
+    if (!staged) HF_CK(cudaStreamSynchronize(C->stream));
     C->par.dt = C->h_ipar[0].dt;
     C->P.par.dt = C->h_ipar[0].dt;
     return HF_OK;
@@ -4198,7 +4294,7 @@ extern "C" int hf_case_instance_failures(hf_case *C, int32_t *status, int32_t n)
         for (int i = 0; i < n; i++) status[i] = 0;
         return HF_OK;
     }
-    int rc = pull_state(C);
+    int rc = want_state(C);
     if (rc) return rc;
     for (int i = 0; i < n; i++) status[i] = C->h_S[i].failed;
     return HF_OK;
@@ -4211,7 +4307,7 @@ extern "C" int hf_case_instance_iters(hf_case *C, int64_t *total_iters, int32_t 
         total_iters[0] = C->stats.total_iters;
         return HF_OK;
     }
-    int rc = pull_state(C);
+    int rc = want_state(C);
     if (rc) return rc;
     for (int i = 0; i < n; i++) total_iters[i] = C->h_S[i].total_iters;
     return HF_OK;
@@ -4293,8 +4389,11 @@ extern "C" void hf_case_destroy(hf_case *C)
         if (C->ev[k]) cudaEventDestroy(C->ev[k]);
     for (void *p : C->owned) cudaFreeAsync(p, C->stream);
     delete C->h_scal;
-    delete[] C->h_S;
-    delete C->h_ctl;
+    if (!C->state_pinned) {
+        delete[] C->h_S;
+        delete C->h_ctl;
+    }
+    pinned_pool().give(C->pin);
     for (cudaStream_t q : C->solve_streams) cudaStreamDestroy(q);
     for (cudaEvent_t q : C->solve_events) cudaEventDestroy(q);
     if (C->body_stream) cudaStreamDestroy(C->body_stream);
