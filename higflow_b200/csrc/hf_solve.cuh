@@ -448,6 +448,9 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_solve(PcgFine G, SolveArgs
     const int lg_r = I.lg_r;
     int lg_d = 5;   // threads per row of the dense solve (log2)
     while (lg_d > 0 && (I.nc << lg_d) > nt) lg_d--;
+    // (a slice's padding multiplies element 0 of shared memory, the first of cvec,
+    // by zero: it has to be a number before the first way down)
+    if (tid == 0) at<T>(cb) = T(0);
     // every CTA of the cluster has started (its shared memory may be written)
     solve::team_sync(t);
 
