@@ -2098,7 +2098,7 @@ int build_pcg(hf_case *C, const std::vector<int32_t> &mptr, const std::vector<in
                 std::vector<double> inv;
                 if (!hf::dense_inverse(last.A, inv)) { ih.err = "singular coarsest AMG level"; continue; }
                 ih.inv = std::move(inv);
-                if (C->use_cg && !C->sie && n <= kSolveMaxRows) ih.F = solve::build(ih.H, C->P.ncell);
+                if (C->use_cg && !C->sie && n <= kSolveMaxRows) ih.F = solve::build(ih.H, ih.inv, C->P.ncell);
             }
         };
         const unsigned nt = std::max(1u, std::min(std::thread::hardware_concurrency(), 32u));
@@ -2479,8 +2479,9 @@ int build_pcg(hf_case *C, const std::vector<int32_t> &mptr, const std::vector<in
         std::vector<const solve::HostSolve *> F(ni);
         for (int i = 0; i < ni; i++) {
             F[i] = &IH[i].F;
-            C->coarse_rows += F[i]->nc;
-            C->coarse_dense += (int64_t)F[i]->nc * F[i]->nc;
+            const int64_t cn = IH[i].H[clev[i]].A.n;
+            C->coarse_rows += cn;
+            C->coarse_dense += cn * cn;
         }
         const int rc = mixed ? build_solve<float>(C, K32, F, C->si32) : build_solve<double>(C, K64, F, C->si64);
         if (rc) return rc;

@@ -77,6 +77,7 @@ struct SOp {
 struct SRank {
     SOp down[kMaxLevels];     // Rt of level l (rows: the next level's)
     SOp up[kMaxLevels];       // Mt and Pt of level l > 0 together; the finest level: Pt
+    SOp coarse;               // the coarsest levels' operator (SInst::dist)
     STab desc0;               // finest level's own rows: uint2 {Pt template row, Pt anchor (element index) << 16 | Mt/A template}
     STab desc_r;              // template form of the first way down: uint2 {Rt template row, anchor (element index)}
 };
@@ -84,6 +85,8 @@ struct SRank {
 template <typename T>
 struct SInst {
     int32_t inst, row0, n, clev, nc;         // clev: the coarsest level; nc: its rows
+    int32_t ndown, ncb;                      // operators down; rows the last of them writes (cvec; nc results follow)
+    int32_t dist;                            // 0: dense inverse in every CTA; 1: SRank::coarse, rows shared out
     int32_t tpl_p, tpl_r, lg_r;              // the finest Pt / Rt as templates; threads per Rt row (log2)
     uint32_t vr, vq, vz, vp, vx;             // finest vectors in shared memory (bytes; vx: x, or e in the mixed form)
     uint32_t vb[kMaxLevels], vo[kMaxLevels]; // vectors of the levels between (bytes)
@@ -327,7 +330,7 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_solve(PcgFine G, SolveArgs
     using solve::at;
     __shared__ SInst<T> I;
     __shared__ SRank Rk;
-    __shared__ solve::Op od[kMaxLevels], ou[kMaxLevels];
+    __shared__ solve::Op od[kMaxLevels], ou[kMaxLevels], ocoarse;
     __shared__ solve::Vec<T> vb[kMaxLevels], vo[kMaxLevels];
     __shared__ __align__(16) double slot[2][kSolveMaxCluster];
     __shared__ double warp_sums[kSolveWarps];
@@ -372,6 +375,7 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_solve(PcgFine G, SolveArgs
         load(Rk.down[l].t, rt);
         load(Rk.up[l].t, rt);
     }
+    if (I.dist) load(Rk.coarse.t, rt);
     auto vec = [&](int id, uint32_t off, int rows) {
         solve::Vec<T> v;
         const int4 g = rng[id][t.rank];
@@ -394,6 +398,7 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_solve(PcgFine G, SolveArgs
         const uint32_t b = o.t.s != kSolveGlobal ? o.t.s : 0u;
         return solve::Op{o.t.s != kSolveGlobal ? nullptr : rt + o.t.g, b, b + o.val, b + o.idx, o.row0, o.rows, o.lg, o.nsl};
     };
+    if (tid == 0) ocoarse = resolve(Rk.coarse);
     if (tid < clev) {
         od[tid] = resolve(Rk.down[tid]);
         ou[tid] = resolve(Rk.up[tid]);
@@ -438,10 +443,13 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_solve(PcgFine G, SolveArgs
     for (int i = xlo + tid; i < xhi; i += nt) at<T>(r.row(i)) = A.r[I.row0 + i];
     const uint32_t tabA = I.a.s, tabM = I.m.s, desc = Rk.desc0.s - 8u * (uint32_t)lo;
     const int kk = K > 0 ? K : kf;
-    const uint32_t cb = I.cvec, co = cb + (uint32_t)I.nc * kT, cb_sh = solve::address(solve::dyn + cb);
+    const uint32_t cb = I.cvec, co = cb + (uint32_t)I.ncb * kT, cb_sh = solve::address(solve::dyn + cb),
+                   co_sh = solve::address(solve::dyn + co);
+    const int ndown = I.ndown;
+    const bool dist = I.dist != 0;
     // the first way down in template form: own rows
     int ra, rh;
-    solve::rank_rows(t.rank, t.size, clev == 1 ? I.nc : clev > 1 ? I.lvl[1] : 0, ra, rh);
+    solve::rank_rows(t.rank, t.size, ndown == 1 ? I.ncb : ndown > 1 ? I.lvl[1] : 0, ra, rh);
     const uint32_t desc_r = Rk.desc_r.s - 8u * (uint32_t)ra;
     const bool tpl_p = I.tpl_p != 0, tpl_r = I.tpl_r != 0;
     const uint32_t tpv = I.tpv.s, tpo = I.tpo.s, trv = I.trv.s, tro = I.tro.s;
@@ -477,21 +485,21 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_solve(PcgFine G, SolveArgs
         }
         __syncthreads();
     };
-    // rows of the coarsest level: to every CTA
-    auto to_all = [&](int i, T v, int lane, int lanes) {
+    // rows of the coarsest vectors: to every CTA
+    auto to_all = [&](uint32_t sh, uint32_t own, int i, T v, int lane, int lanes) {
         if (t.size > 1) {
-            for (int k = lane; k < t.size; k += lanes) solve::store_peer(solve::peer(cb_sh + i * kT, k), v);
+            for (int k = lane; k < t.size; k += lanes) solve::store_peer(solve::peer(sh + i * kT, k), v);
         } else if (lane == 0) {
-            at<T>(cb + i * kT) = v;
+            at<T>(own + i * kT) = v;
         }
     };
     // the way down from level l: b_{l+1} = Rt b_l
     auto down = [&](int l) {
-        const bool last = l + 1 == clev;
+        const bool last = l + 1 == ndown;
         const solve::Vec<T> nb = vb[last ? l : l + 1];
         const int lg = od[l].lg;
         solve::apply<T>(od[l], [&](int i, T v, int lane) {
-            if (last) to_all(i, v, lane, 1 << lg);
+            if (last) to_all(cb_sh, cb, i, v, lane, 1 << lg);
             else if (lane == 0) nb.put(i, v);
         });
     };
@@ -505,7 +513,7 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_solve(PcgFine G, SolveArgs
             down(0);
             return;
         }
-        const bool last = clev == 1;
+        const bool last = ndown == 1;
         const solve::Vec<T> nb = vb[1];
         const int lanes = 1 << lg_r, lane = tid & (lanes - 1), step = nt >> lg_r;
         for (int b = ra; b < rh; b += step) {
@@ -513,7 +521,7 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_solve(PcgFine G, SolveArgs
             const uint2 d = i < rh ? at<uint2>(desc_r + 8u * i) : make_uint2(0u, 0u);
             const T s = solve::lanes_sum(solve::row_part<T>(trv, tro, d.x, lane, lanes, d.y * kT), lanes);
             if (i < rh) {
-                if (last) to_all(i, s, lane, lanes);
+                if (last) to_all(cb_sh, cb, i, s, lane, lanes);
                 else if (lane == 0) nb.put(i, s);
             }
         }
@@ -522,11 +530,17 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_solve(PcgFine G, SolveArgs
     // b_1, and has not yet on z)
     auto vcycle = [&]() -> double {
         double part = 0.0;
-        for (int l = 1; l < clev; l++) {
+        for (int l = 1; l < ndown; l++) {
             down(l);
             solve::team_sync(t);
         }
-        dense();
+        if (dist) {
+            const int lg = ocoarse.lg;
+            solve::apply<T>(ocoarse, [&](int i, T v, int lane) { to_all(co_sh, co, i, v, lane, 1 << lg); });
+            solve::team_sync(t);
+        } else {
+            dense();
+        }
         for (int l = clev - 1; l > 0; l--) {
             const solve::Vec<T> ol = vo[l];
             solve::apply<T>(ou[l], [&](int i, T v, int lane) { if (lane == 0) ol.put(i, v); });
@@ -821,6 +835,14 @@ struct HostSolve {
     };
     std::vector<Level> L;
     std::vector<int> cpos;      // the coarsest level's rows: their places here (empty: unchanged)
+    // The coarsest levels as one dense operator, its rows shared out over the
+    // ranks (row-major, nc x ncb); empty: the coarsest level's inverse in every
+    // CTA.  g false: the whole V-cycle from level clev's b to its out, Mt + Pt
+    // inverse Rt of that level and the one below it; g true: inverse Rt, from
+    // level clev - 1's b to the coarsest level's out.
+    std::vector<double> coarse;
+    bool g = false;
+    int ndown = 0, ncb = 0;
     // finest level: A and Mt as templates of `fine` entries, per row the template
     std::vector<uint32_t> tpl;
     std::vector<int32_t> off;
@@ -872,6 +894,7 @@ inline void ranges(HostSolve &S)
             for (int k = 0; k < S.fine; k++) grow(g, i + S.off[(size_t)S.tpl[i] * S.fine + k]);
     };
     const int levels = std::max(1, S.clev);   // levels with distributed vectors
+    auto whole = [&](int l) { return S.g && l == S.clev - 1; };   // b: the coarse operator's input, held by all
     for (int l = 0; l < levels; l++) {
         const HostSolve::Level &L = S.L[l];
         for (int k = 0; k < C; k++) {
@@ -882,7 +905,10 @@ inline void ranges(HostSolve &S)
             b = make_int4(lo, hi, k, k);
             if (l == 0) reach_fine(b, lo, hi);
             else reach(b, L.m, lo, hi);
-            if (l < S.clev) {
+            if (whole(l)) {
+                b.x = 0;
+                b.y = L.n;
+            } else if (l < S.clev) {
                 rank_rows(k, C, rows(l + 1), a, h);
                 reach(b, L.r, a, h);
             }
@@ -915,7 +941,49 @@ inline void ranges(HostSolve &S)
         }
 }
 
-inline HostSolve build(const std::vector<hf::HostLevel> &H, long total)
+// The coarsest levels as one dense operator where a rank's rows of it are small
+// (kSolveCoarse bytes): one phase and no replicated dense solve, in place of two
+// to three phases.
+constexpr size_t kSolveCoarse = 76 * 1024;
+inline void coarse_operator(HostSolve &S, const std::vector<double> &inverse)
+{
+    const int last = S.clev - 1, n = S.L[last].n, nc = S.nc, C = S.cluster;
+    const HostSolve::Level &L = S.L[last];
+    auto bytes = [&](int rows) { return (size_t)((rows + C - 1) / C) * n * 10; };
+    if (bytes(nc) > kSolveCoarse) return;
+    // G = inverse Rt (rows and columns in this file's order)
+    std::vector<int> old(nc);
+    for (int i = 0; i < nc; i++) old[S.cpos.empty() ? i : S.cpos[i]] = i;
+    std::vector<double> G((size_t)nc * n, 0.0);
+    for (int i = 0; i < nc; i++)
+        for (int j = 0; j < nc; j++) {
+            const double v = inverse[(size_t)old[i] * nc + old[j]];
+            for (int k = L.r.ptr[j]; k < L.r.ptr[j + 1]; k++) G[(size_t)i * n + L.r.col[k]] += v * L.r.val[k];
+        }
+    if (bytes(n) > kSolveCoarse) {
+        S.g = true;
+        S.coarse = std::move(G);
+        S.ndown = last;
+        S.ncb = n;
+        return;
+    }
+    // Mt + Pt G
+    S.coarse.assign((size_t)n * n, 0.0);
+    for (int i = 0; i < n; i++) {
+        double *row = S.coarse.data() + (size_t)i * n;
+        for (int k = L.m.ptr[i]; k < L.m.ptr[i + 1]; k++) row[L.m.col[k]] += L.m.val[k];
+        for (int k = L.p.ptr[i]; k < L.p.ptr[i + 1]; k++) {
+            const double *g = G.data() + (size_t)L.p.col[k] * n;
+            for (int j = 0; j < n; j++) row[j] += L.p.val[k] * g[j];
+        }
+    }
+    S.clev = S.ndown = last;
+    S.nc = S.ncb = n;
+    S.L.resize(last);
+    S.cpos.clear();
+}
+
+inline HostSolve build(const std::vector<hf::HostLevel> &H, const std::vector<double> &inverse, long total)
 {
     HostSolve S;
     S.clev = (int)H.size() - 1;
@@ -979,6 +1047,9 @@ inline HostSolve build(const std::vector<hf::HostLevel> &H, long total)
         else S.cpos = pos;
         fine_pos = std::move(pos);
     }
+    S.ndown = S.clev;
+    S.ncb = S.nc;
+    if (S.clev > 1) coarse_operator(S, inverse);
     ranges(S);
     S.ok = true;
     return S;
@@ -1004,6 +1075,9 @@ Packed<T> pack(const HostSolve &S, const std::vector<double> &inverse, bool mixe
     o.n = S.L[0].n;
     o.clev = S.clev;
     o.nc = S.nc;
+    o.ndown = S.ndown;
+    o.ncb = S.ncb;
+    o.dist = !S.coarse.empty();
     for (int l = 0; l < (int)S.L.size(); l++) o.lvl[l] = S.L[l].n;
     size_t at = 0;
     auto round = [](size_t b) { return (b + 15) & ~size_t(15); };
@@ -1015,11 +1089,11 @@ Packed<T> pack(const HostSolve &S, const std::vector<double> &inverse, bool mixe
     };
     // the vectors that are gathered from or exchanged always live in shared
     // memory, at element indices of 16 bits
-    o.cvec = take(sizeof(T) * 2 * S.nc);
+    o.cvec = take(sizeof(T) * (S.ncb + S.nc));
     o.vr = take(sizeof(T) * S.held[0]);
     o.vz = take(sizeof(T) * S.held[1]);
     for (int l = 1; l < S.clev; l++) {
-        o.vb[l] = take(sizeof(T) * S.held[2 * l]);
+        o.vb[l] = S.g && l == S.clev - 1 ? o.cvec : take(sizeof(T) * S.held[2 * l]);
         o.vo[l] = take(sizeof(T) * S.held[2 * l + 1]);
         if (o.vb[l] == kSolveGlobal || o.vo[l] == kSolveGlobal) return K;
     }
@@ -1061,7 +1135,7 @@ Packed<T> pack(const HostSolve &S, const std::vector<double> &inverse, bool mixe
     };
     // one operator's rows of every rank in slices; f adds row i's entries
     using Row = std::vector<std::pair<uint16_t, T>>;
-    auto slices = [&](int rows, int lg_max, auto f, SOp (SRank::*arr)[kMaxLevels], int l) {
+    auto slices = [&](int rows, int lg_max, auto f, auto of) {
         size_t most = 0;
         std::vector<std::vector<char>> data(C);
         double entries = 0;
@@ -1084,7 +1158,7 @@ Packed<T> pack(const HostSolve &S, const std::vector<double> &inverse, bool mixe
         for (int k = 0; k < C; k++) {
             int a, h;
             rank_rows(k, C, rows, a, h);
-            SOp &op = (K.ranks[k].*arr)[l];
+            SOp &op = of(K.ranks[k]);
             op.row0 = a;
             op.rows = h - a;
             op.lg = lg;
@@ -1124,7 +1198,7 @@ Packed<T> pack(const HostSolve &S, const std::vector<double> &inverse, bool mixe
         }
         const uint32_t s = take(most);
         for (int k = 0; k < C; k++) {
-            SOp &op = (K.ranks[k].*arr)[l];
+            SOp &op = of(K.ranks[k]);
             op.t.s = s;
             op.t.bytes = (uint32_t)data[k].size();
             op.t.g = blob(K.rank_tables, data[k].data(), data[k].size());
@@ -1135,7 +1209,7 @@ Packed<T> pack(const HostSolve &S, const std::vector<double> &inverse, bool mixe
     };
     // level l's out (the coarsest level's: co)
     auto out_elem = [&](int l, int k, int i) {
-        return l == S.clev ? (uint32_t)(o.cvec / sizeof(T)) + S.nc + i : elem(o.vo[l], 2 * l + 1, k, i);
+        return l == S.clev ? (uint32_t)(o.cvec / sizeof(T)) + S.ncb + i : elem(o.vo[l], 2 * l + 1, k, i);
     };
     auto b_elem = [&](int l, int k, int i) { return l == 0 ? elem(o.vr, 0, k, i) : elem(o.vb[l], 2 * l, k, i); };
     // the finest level's Pt and Rt as templates, where that form is the smaller
@@ -1229,11 +1303,17 @@ Packed<T> pack(const HostSolve &S, const std::vector<double> &inverse, bool mixe
         slices(L.n, 5, [&](int k, int i, Row &row) {
             add(row, L.m, i, [&](int c) { return b_elem(l, k, c); });
             add(row, L.p, i, [&](int c) { return out_elem(l + 1, k, c); });
-        }, &SRank::up, l);
-        slices(L.r.rows(), 5, [&](int k, int i, Row &row) { add(row, L.r, i, [&](int c) { return b_elem(l, k, c); }); },
-               &SRank::down, l);
+        }, [l](SRank &r) -> SOp & { return r.up[l]; });
+        if (l < S.ndown)
+            slices(L.r.rows(), 5, [&](int k, int i, Row &row) { add(row, L.r, i, [&](int c) { return b_elem(l, k, c); }); },
+                   [l](SRank &r) -> SOp & { return r.down[l]; });
     }
-    {
+    if (o.dist) {
+        slices(S.nc, 5, [&](int, int i, Row &row) {
+            for (int j = 0; j < S.ncb; j++)
+                row.emplace_back((uint16_t)(o.cvec / sizeof(T) + j), (T)S.coarse[(size_t)i * S.ncb + j]);
+        }, [](SRank &r) -> SOp & { return r.coarse; });
+    } else {
         std::vector<T> d(inverse.size());
         for (int i = 0; i < S.nc; i++)
             for (int j = 0; j < S.nc; j++)
@@ -1245,10 +1325,10 @@ Packed<T> pack(const HostSolve &S, const std::vector<double> &inverse, bool mixe
         const HostSolve::Level &L = S.L[0];
         if (!o.tpl_r)
             slices(L.r.rows(), 5, [&](int k, int i, Row &row) { add(row, L.r, i, [&](int c) { return b_elem(0, k, c); }); },
-                   &SRank::down, 0);
+                   [](SRank &r) -> SOp & { return r.down[0]; });
         if (!o.tpl_p)
             slices(L.n, 0, [&](int k, int i, Row &row) { add(row, L.p, i, [&](int c) { return out_elem(1, k, c); }); },
-                   &SRank::up, 0);
+                   [](SRank &r) -> SOp & { return r.up[0]; });
     }
     o.vp = take(sizeof(T) * own);
     o.vx = take((mixed ? sizeof(T) : sizeof(double)) * own);
