@@ -50,6 +50,7 @@ struct Team {
     int rank, size, m, nvb;
     double (*wsum)[8];                      // [2 * m]: the warps' sums of the own blocks
     double (*blk)[2][kBiMaxBlocks];         // [2][value][block], double buffered
+    double (*fin)[8];                       // [value]: sums of 32 blocks
     int par;
 };
 
@@ -94,16 +95,17 @@ __device__ __forceinline__ void team_sum(Team &t, double (&tot)[NV])
         else *p = s;
     }
     team_sync(t);
-#pragma unroll
-    for (int v = 0; v < NV; v++) {
-        double c[8];
-#pragma unroll
-        for (int q = 0; q < 8; q++) {
-            c[q] = 0.0;
-            if (32 * q < t.nvb) c[q] = warp_sum(32 * q + lane < t.nvb ? t.blk[t.par][v][32 * q + lane] : 0.0);
-        }
-        tot[v] = __shfl_sync(0xffffffffu, add8(c), 0);
+    // a warp per value and 32 blocks (the sums of blocks that do not exist stay
+    // zero)
+    const int parts = (t.nvb + 31) / 32;
+    for (int k = tid >> 5; k < NV * parts; k += blockDim.x >> 5) {
+        const int v = k / parts, q = k % parts;
+        const double s = warp_sum(32 * q + lane < t.nvb ? t.blk[t.par][v][32 * q + lane] : 0.0);
+        if (lane == 0) t.fin[v][q] = s;
     }
+    __syncthreads();
+#pragma unroll
+    for (int v = 0; v < NV; v++) tot[v] = add8(t.fin[v]);
 }
 
 }  // namespace bicg
@@ -114,6 +116,7 @@ __global__ void __launch_bounds__(kBiThreads, 1) k_bi_solve(const BiArgs *args)
     __shared__ BiSys Y;
     __shared__ double wsum[2 * kBiMaxBlocks / 4][8];
     __shared__ double blk[2][2][kBiMaxBlocks];
+    __shared__ double fin[2][8];
     __shared__ int4 rng[kBiMaxCluster];
     const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31;
     bicg::Team t;
@@ -129,6 +132,8 @@ __global__ void __launch_bounds__(kBiThreads, 1) k_bi_solve(const BiArgs *args)
     t.nvb = (n + kBlock - 1) / kBlock;
     t.wsum = wsum;
     t.blk = blk;
+    t.fin = fin;
+    if (tid < 16) (&fin[0][0])[tid] = 0.0;
     t.par = 0;
     if (tid < t.size) rng[tid] = Y.rng[tid];
     const int lo = min(n, t.rank * rows), own = min(n, lo + rows) - lo;
