@@ -1298,6 +1298,8 @@ Packed<T> pack(const HostSolve &S, const std::vector<double> &inverse, bool mixe
             if (o.tpv.s == kSolveGlobal || o.tpo.s == kSolveGlobal) return K;
         }
     }
+    o.vp = take(sizeof(T) * own);
+    o.vx = take((mixed ? sizeof(T) : sizeof(double)) * own);
     for (int l = S.clev - 1; l > 0; l--) {
         const HostSolve::Level &L = S.L[l];
         slices(L.n, 5, [&](int k, int i, Row &row) {
@@ -1330,8 +1332,6 @@ Packed<T> pack(const HostSolve &S, const std::vector<double> &inverse, bool mixe
             slices(L.n, 0, [&](int k, int i, Row &row) { add(row, L.p, i, [&](int c) { return out_elem(1, k, c); }); },
                    [](SRank &r) -> SOp & { return r.up[0]; });
     }
-    o.vp = take(sizeof(T) * own);
-    o.vx = take((mixed ? sizeof(T) : sizeof(double)) * own);
     if (mixed) {
         std::vector<SEnt<double>> e(S.off.size());
         for (size_t q = 0; q < e.size(); q++) e[q] = SEnt<double>{S.va[q], S.off[q], 0};
