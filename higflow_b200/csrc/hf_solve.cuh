@@ -36,7 +36,7 @@
 
 constexpr int kSolveThreads = 1024;          // most threads of a CTA
 constexpr int kSolveWarps = kSolveThreads / 32;
-constexpr int kSolveSmem = 208 * 1024;       // dynamic shared memory
+constexpr int kSolveSmem = 213 * 1024;       // dynamic shared memory (227 KB less the static part)
 constexpr int kSolveLenBits = 10;            // template rows of up to 1023 entries, 2^22 entries per operator
 constexpr int kSolveMaxCluster = 16;
 constexpr int kSolveVecs = 2 * kMaxLevels;   // vectors with halos: r (and q), z, then b and out of the levels between
@@ -941,9 +941,11 @@ inline void ranges(HostSolve &S)
         }
 }
 
-// The coarsest levels as one dense operator where a rank's rows of it are small
-// (kSolveCoarse bytes): one phase and no replicated dense solve, in place of two
-// to three phases.
+// The coarsest levels as one dense operator where a rank's rows of it are small:
+// one phase and no replicated dense solve, in place of two to three phases.  The
+// square form up to half of kSolveCoarse bytes (beyond that it displaces finer
+// operators from shared memory: 129 x 129 FP64 228 us a step with it, 214 with
+// inverse Rt alone), inverse Rt up to kSolveCoarse.
 constexpr size_t kSolveCoarse = 76 * 1024;
 inline void coarse_operator(HostSolve &S, const std::vector<double> &inverse)
 {
@@ -960,7 +962,7 @@ inline void coarse_operator(HostSolve &S, const std::vector<double> &inverse)
             const double v = inverse[(size_t)old[i] * nc + old[j]];
             for (int k = L.r.ptr[j]; k < L.r.ptr[j + 1]; k++) G[(size_t)i * n + L.r.col[k]] += v * L.r.val[k];
         }
-    if (bytes(n) > kSolveCoarse) {
+    if (bytes(n) > kSolveCoarse / 2) {
         S.g = true;
         S.coarse = std::move(G);
         S.ndown = last;
@@ -1031,12 +1033,29 @@ inline HostSolve build(const std::vector<hf::HostLevel> &H, const std::vector<do
         const hf::HostLevel &h = H[l];
         const int nn = h.R.n;
         std::vector<std::pair<double, int>> key(nn);
-        for (int i = 0; i < nn; i++) {
-            double sum = 0.0;
-            const int a = h.R.ptr[i], e = h.R.ptr[i + 1];
-            for (int k = a; k < e; k++) sum += l == 0 ? h.R.col[k] : fine_pos[h.R.col[k]];
-            key[i] = {e > a ? sum / (e - a) : 0.0, i};
-        }
+        double run = 0.0, span = 0.0;
+        for (int pass = 0; pass < 2; pass++)
+            for (int i = 0; i < nn; i++) {
+                double sum = 0.0, lo = h.A.n, hi = 0.0;
+                const int a = h.R.ptr[i], e = h.R.ptr[i + 1];
+                for (int k = a; k < e; k++) {
+                    const double c = l == 0 ? h.R.col[k] : fine_pos[h.R.col[k]];
+                    sum += c;
+                    lo = std::min(lo, c);
+                    hi = std::max(hi, c);
+                }
+                if (pass == 0) {
+                    span = std::max(span, hi - lo);
+                    continue;
+                }
+                // rows that follow their predecessors keep their order (and the
+                // regular numbering that makes rows share templates); a row far
+                // behind them goes to its place
+                const double mean = e > a ? sum / (e - a) : 0.0;
+                const bool in_order = mean + span >= run;
+                if (in_order) run = std::max(run, mean);
+                key[i] = {in_order ? run : mean, i};
+            }
         std::sort(key.begin(), key.end());
         std::vector<int> pos(nn);
         for (int i = 0; i < nn; i++) pos[key[i].second] = i;
