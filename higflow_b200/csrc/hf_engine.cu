@@ -1986,10 +1986,13 @@ constexpr int kSolveMaxRows = 1 << 19;
 // The one-launch solves' tables of every instance on the device, the instances
 // grouped by cluster size (one launch each), largest first.
 template <typename T>
-auto solve_kernel(int fine) -> void (*)(PcgFine, SolveArgs<T>, int)
+auto solve_kernel(int fine, int threads) -> void (*)(PcgFine, SolveArgs<T>, int)
 {
     constexpr bool mix = std::is_same<T, float>::value;
-    return fine == 5 ? k_solve<T, mix, 5> : fine == 7 ? k_solve<T, mix, 7> : k_solve<T, mix, 0>;
+    if (threads <= 512)
+        return fine == 5 ? k_solve<T, mix, 5, 512> : fine == 7 ? k_solve<T, mix, 7, 512> : k_solve<T, mix, 0, 512>;
+    return fine == 5 ? k_solve<T, mix, 5, kSolveThreads>
+                     : fine == 7 ? k_solve<T, mix, 7, kSolveThreads> : k_solve<T, mix, 0, kSolveThreads>;
 }
 
 template <typename T>
@@ -2038,7 +2041,7 @@ int build_solve(hf_case *C, std::vector<solve::Packed<T>> &K, const std::vector<
         size_t most = 0;
         for (; e < ni && key(order[e]) == key(order[k]); e++) most = std::max(most, K[order[e]].smem);
         C->solves.push_back(hf_case::SolveLaunch{k, e - k, f.cluster, f.fine, f.threads, most});
-        auto *kern = solve_kernel<T>(f.fine);
+        auto *kern = solve_kernel<T>(f.fine, f.threads);
         HF_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSolveSmem));
         HF_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
         k = e;
@@ -2688,9 +2691,9 @@ int enqueue_solve(hf_case *C, cudaStream_t st, int &kernels)
         kernels++;
         const PcgFine &G = C->G;
         if (C->mixed)
-            return cudaLaunchKernelEx(&cfg, solve_kernel<float>(L.fine), G,
+            return cudaLaunchKernelEx(&cfg, solve_kernel<float>(L.fine, L.threads), G,
                                       SolveArgs<float>{C->si32, G.r32, C->pa32, G.e32, L.first}, L.fine);
-        return cudaLaunchKernelEx(&cfg, solve_kernel<double>(L.fine), G,
+        return cudaLaunchKernelEx(&cfg, solve_kernel<double>(L.fine, L.threads), G,
                                   SolveArgs<double>{C->si64, G.r, C->pa, nullptr, L.first}, L.fine);
     };
     if (C->solves.size() > 1) HF_CK(cudaEventRecord(C->solve_events[0], st));

@@ -323,9 +323,11 @@ __device__ __forceinline__ void apply(const Op &O, Put put)
 
 }  // namespace solve
 
-// K: entries of the finest operator's rows (5: 2D, 7: 3D uniform grids), 0: see kf
-template <typename T, bool MIX, int K>
-__global__ void __launch_bounds__(kSolveThreads, 1) k_solve(PcgFine G, SolveArgs<T> A, int kf)
+// K: entries of the finest operator's rows (5: 2D, 7: 3D uniform grids), 0: see
+// kf.  NT: most threads of a CTA; 512 leave a thread 128 registers instead of 64
+// (Poisson solve per step: 1,089 rows 131 -> 126 us, 4,913 rows in 3D 183 -> 177)
+template <typename T, bool MIX, int K, int NT>
+__global__ void __launch_bounds__(NT, 1) k_solve(PcgFine G, SolveArgs<T> A, int kf)
 {
     using solve::at;
     __shared__ SInst<T> I;
@@ -866,13 +868,15 @@ inline int cluster_size(int n, long total)
 
 // Threads of a CTA with `own` rows of the finest level: the fewest turns a full
 // block needs, and no more warps than these turns take (every warp pays a
-// phase's fixed instructions).  The instances of a batch share three sizes, so
-// that few launches cover them.
+// phase's fixed instructions); of 512 threads up to kSolveSmall rows, where the
+// registers are worth more than the threads.  The instances of a batch share
+// three sizes, so that few launches cover them.
+constexpr int kSolveSmall = 1536;
 inline int block_threads(int own, bool batch)
 {
     if (batch) return own <= 256 ? 256 : own <= 512 ? 512 : kSolveThreads;
-    const int turns = (own + kSolveThreads - 1) / kSolveThreads;
-    return std::min(kSolveThreads, std::max(128, ((own + turns - 1) / turns + 31) / 32 * 32));
+    const int most = own <= kSolveSmall ? 512 : kSolveThreads, turns = (own + most - 1) / most;
+    return std::min(most, std::max(128, ((own + turns - 1) / turns + 31) / 32 * 32));
 }
 
 // the rows of every vector that each rank holds: its own and the columns its
