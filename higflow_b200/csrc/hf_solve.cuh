@@ -12,8 +12,9 @@
 //      b_{l+1} = Rt b_l,  Rt = R (I - A w D^-1)   (pre-smoothing, residual, R)
 //      out_l = Mt b_l + Pt out_{l+1},  Mt = 2 w D^-1 - w D^-1 A w D^-1,
 //      Pt = (I - w D^-1 A) P                      (prolongation, post-smoothing)
-//    (the same V-cycle in exact arithmetic); the dense coarsest solve runs in
-//    every CTA for itself;
+//    (the same V-cycle in exact arithmetic); the coarsest levels are one dense
+//    operator with its rows shared out over the CTAs where it is small, else
+//    the dense solve runs in every CTA for itself;
 //  - q = A p is carried as q = A z + beta q, so p has no neighbour reads, and r
 //    is updated over a CTA's halo as well as its own rows from the halo of q, so
 //    the update and the first phase down need no barrier between them;
@@ -66,7 +67,8 @@ struct STab {
 // An operator's rows of one rank as slices: slice k holds 32 >> lg rows, 1 << lg
 // threads each; the entries of its 32 threads lie side by side, turn by turn
 // (turns ptr[k] to ptr[k + 1]).  t: ptr (padded to 16 bytes), the values, the
-// columns (16-bit element indices into shared memory).
+// columns (16-bit element indices into shared memory).  Padding is value 0 at
+// element 0, which k_solve sets to a number first.
 struct SOp {
     STab t;
     int32_t row0, rows, lg, nsl;
@@ -854,8 +856,8 @@ struct HostSolve {
 // CTAs of an instance's cluster: about kSolveRows rows each while the case's
 // instances leave SMs idle (a phase then takes one row per thread or less and
 // its latency counts), up to 4096 when they fill the device anyway.  Measured,
-// Poisson solve per step: 4,096 rows alone (FP64) 150 / 148 / 170 / 255 us at
-// 256 / 512 / 1024 / 2048 rows a CTA, 4,913 rows in 3D 209 / 210 / 273 / 354.
+// Poisson solve per step: 4,096 rows alone (FP64) 135 / 137 / 181 us at
+// 256 / 512 / 1024 rows a CTA, 4,913 rows in 3D 184 / 183 / 240.
 constexpr int kSolveRows = 512;
 inline int cluster_size(int n, long total)
 {
