@@ -67,3 +67,29 @@ def test_semi_implicit_steps_match_64_bit_steps(sides):
         err = np.linalg.norm(got[k] - w) / np.linalg.norm(w)
         assert err < (1e-7 if k == "p" else 1e-10), f"{k}: {err:.2e}"
     c.close()
+
+
+# clusters smaller than alone (over 148 * 512 rows in all), and instances that
+# run in a cluster alone but in the level-synchronous loop beside a larger one
+@pytest.mark.parametrize("sides", ["219,155,64,129,33", "460,33,9"])
+def test_instances_alone_and_in_a_batch_that_splits_them_otherwise(sides):
+    case = dict(flow="newtonian", sides=sides, steps=3, precision="plain", scheme="explicit", per_step=False, limits="")
+    progs = cases._programs(case)
+    parts, whole = cases._inputs(case, 7)
+
+    def stepped(prog, fields):
+        c = engine.Case(prog, engine.options(precision=hp.PREC_FP64, rtol=1e-13, atol=1e-300))
+        for (fid, comp), v in fields.items():
+            c.set(fid, comp, v)
+        c.step(3)
+        return c
+
+    batch = stepped(hp.Program.concatenate(progs), whole)
+    for i, prog in enumerate(progs):
+        alone = stepped(prog, parts[i])
+        for fid, comp in ((hp.FIELD_U, 0), (hp.FIELD_U, 1), (hp.FIELD_P, 0)):
+            a = alone.get(fid, comp)
+            err = np.linalg.norm(batch.get_instance(fid, comp, i) - a) / np.linalg.norm(a)
+            assert err < 1e-10, (i, fid, comp, err)
+        alone.close()
+    batch.close()
