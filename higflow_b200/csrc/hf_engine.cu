@@ -3245,6 +3245,7 @@ int graph_steps(hf_case *C, int nsteps, bool sync)
     if (rc) return rc;
     const bool ve = C->par.flowtype == HF_VISCOELASTIC;
     auto one = [&]() -> int {
+        C->state_fresh = false;   // (with profiling on, the step before was just fetched)
         if (eager) return eager_step<D>(C);
         HF_CK(cudaGraphLaunch(C->exec[ve ? C->parity : 0], C->stream));
         return HF_OK;
@@ -3371,7 +3372,6 @@ int bicg_step(hf_case *C)
 
 int run_steps(hf_case *C, int nsteps, bool sync)
 {
-    if (nsteps > 0) C->state_fresh = false;
     if (!C->use_cg) {
         for (int s = 0; s < nsteps; s++) {
             int rc = C->D == 2 ? bicg_step<2>(C) : bicg_step<3>(C);
