@@ -1553,6 +1553,7 @@ struct hf_case {
     size_t stage0 = 0, stage_at = 0;
     bool state_pinned = false;
     bool state_fresh = false;       // the mirrors hold the state after the last step
+    bool in_flight = false;         // steps were queued since the stream was last waited for
     cudaStream_t body_stream = nullptr;
     cudaGraph_t graph[2] = {};
     cudaGraphExec_t exec[2] = {};
@@ -3171,6 +3172,17 @@ int pull_state(hf_case *C)
     HF_CK(cudaStreamSynchronize(C->stream));
     C->stage_at = C->stage0;
     C->state_fresh = true;
+    C->in_flight = false;
+    return HF_OK;
+}
+
+// waits for the steps queued so far, whose errors the caller then reports
+int settle(hf_case *C)
+{
+    if (!C->in_flight) return HF_OK;
+    HF_CK(cudaStreamSynchronize(C->stream));
+    C->stage_at = C->stage0;
+    C->in_flight = false;
     return HF_OK;
 }
 
@@ -3246,6 +3258,7 @@ int graph_steps(hf_case *C, int nsteps, bool sync)
     const bool ve = C->par.flowtype == HF_VISCOELASTIC;
     auto one = [&]() -> int {
         C->state_fresh = false;   // (with profiling on, the step before was just fetched)
+        C->in_flight = true;
         if (eager) return eager_step<D>(C);
         HF_CK(cudaGraphLaunch(C->exec[ve ? C->parity : 0], C->stream));
         return HF_OK;
@@ -3373,6 +3386,7 @@ int bicg_step(hf_case *C)
 int run_steps(hf_case *C, int nsteps, bool sync)
 {
     if (!C->use_cg) {
+        C->in_flight = true;
         for (int s = 0; s < nsteps; s++) {
             int rc = C->D == 2 ? bicg_step<2>(C) : bicg_step<3>(C);
             if (rc) return rc;
@@ -4080,6 +4094,8 @@ extern "C" int hf_case_set_field(hf_case *C, int32_t field, int32_t comp, const 
     int64_t m = 0;
     double *p = field_ptr(C, field, comp, &m);
     if (!p || m != n) return fail(HF_ERR_INVALID, "field/component/size mismatch");
+    const int rc = settle(C);
+    if (rc) return rc;
     char *staged = stage(C, sizeof(double) * (size_t)n);
     if (staged) memcpy(staged, host, sizeof(double) * (size_t)n);
     HF_CK(cudaMemcpyAsync(p, staged ? (const void *)staged : host, sizeof(double) * (size_t)n, cudaMemcpyHostToDevice, C->stream));
@@ -4235,6 +4251,8 @@ extern "C" int hf_case_set_timestep(hf_case *C, const double *dt, int32_t n)
         if (same) return HF_OK;
         return fail(HF_ERR_UNSUPPORTED, "new time step with the semi-implicit velocity (its matrix holds dt)");
     }
+    const int rc = settle(C);
+    if (rc) return rc;
     // (the parameters go to the device on every call, as the host's dt of
     // each step, in the order of the case stream)
     for (int i = 0; i < n; i++) C->h_ipar[i].dt = dt[i];

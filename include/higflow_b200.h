@@ -310,7 +310,11 @@ typedef struct hf_stats {
 
 /* Replaces higflow_solver_step / _viscoelastic for one case.
  * hf_case_create copies the program to the device; the program memory can be
- * freed afterwards.  Fields start at zero; set them with hf_case_set_field. */
+ * freed afterwards.  Fields start at zero; set them with hf_case_set_field.
+ * hf_case_set_field waits for the steps queued before it; the host array may
+ * be changed or freed as soon as it returns, the copy of a field up to 256 KB
+ * being then still in the case stream's order (later steps see it).
+ * hf_case_get_field waits for everything queued before it. */
 int  hf_case_create(const hf_program *prog, const hf_options *opt, hf_case **out);
 int  hf_case_set_field(hf_case *c, int32_t field, int32_t comp, const double *host, int64_t n);
 int  hf_case_get_field(hf_case *c, int32_t field, int32_t comp, double *host, int64_t n);
@@ -365,7 +369,8 @@ int  hf_case_adjust_timestep(hf_case *c, double *cfl, double *dt, int32_t n);
 /* Set each instance's time step (n = ninst) for the next steps, as a case main
  * loop does when it changes ns->par.dt (higflow_adjust_timestep,
  * hig-flow-timestep.c:115-139, or a restart); the instances' parameters go to
- * the device on every call (it waits for the case's stream).
+ * the device on every call (it waits for the steps queued on the case's
+ * stream; the parameters follow in stream order).
  * HF_ERR_UNSUPPORTED for the semi-implicit velocity when dt changes (its
  * system matrix holds dt; an unchanged dt is accepted and not copied). */
 int  hf_case_set_timestep(hf_case *c, const double *dt, int32_t n);

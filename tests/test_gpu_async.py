@@ -2,6 +2,7 @@
 return and wait for."""
 import numpy as np
 import pytest
+import torch
 
 from higflow_b200 import engine
 from higflow_b200 import program as hp
@@ -57,4 +58,23 @@ def test_failure_of_a_queued_step_is_seen_under_profiling():
     with pytest.raises(engine.EngineError) as e:
         case.synchronize()
     assert e.value.code == -4
+    case.close()
+
+
+@pytest.mark.parametrize("call", ["set_timestep", "set_field"])
+def test_writing_calls_wait_for_the_steps_queued_before_them(call):
+    """hf_case_set_timestep and hf_case_set_field wait for the case's queued
+    steps, so that an error of theirs is not left to a later call."""
+    case, prog = _case()
+    case.step(1)
+    u = case.get(hp.FIELD_U, 0)
+    case.step(1000, sync=False)
+    done = torch.cuda.Event()
+    done.record(torch.cuda.ExternalStream(case.stream()))
+    assert not done.query()
+    if call == "set_timestep":
+        case.set_timestep(prog.par["dt"])
+    else:
+        case.set(hp.FIELD_U, 0, u)
+    assert done.query()
     case.close()
