@@ -1477,6 +1477,55 @@ PinnedPool &pinned_pool()
     return *p;
 }
 
+// How many clusters of this launch the device can hold at once; 0: it cannot be
+// launched at all (16 CTAs of one SM each may be more than a partition's GPCs
+// have), and the caller keeps to kernels without clusters.  An exported function
+// of its own, so that a test can put one without clusters in its place.
+extern "C" int hf_clusters_that_fit(const void *kernel, const cudaLaunchConfig_t *cfg)
+{
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kernel, cfg) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return n;
+}
+
+// a launch of whole clusters
+struct ClusterLaunch {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[2];
+    ClusterLaunch(int clusters, int size, int threads, size_t smem, cudaStream_t st)
+    {
+        cfg.gridDim = dim3((unsigned)(clusters * size));
+        cfg.blockDim = dim3((unsigned)threads);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = st;
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = (unsigned)size;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+    }
+    ClusterLaunch(const ClusterLaunch &) = delete;
+    // programmatic launch behind the kernel it follows on its stream
+    void early()
+    {
+        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[1].val.programmaticStreamSerializationAllowed = 1;
+        cfg.numAttrs = 2;
+    }
+    bool fits(const void *kernel, int smem_most) const
+    {
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_most) != cudaSuccess ||
+            cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        return hf_clusters_that_fit(kernel, &cfg) > 0;
+    }
+};
+
 struct hf_case {
     hf_options opt;
     hf_params par;
@@ -1996,11 +2045,14 @@ auto solve_kernel(int fine, int threads) -> void (*)(PcgFine, SolveArgs<T>, int)
                      : fine == 7 ? k_solve<T, mix, 7, kSolveThreads> : k_solve<T, mix, 0, kSolveThreads>;
 }
 
+// The instances in the order of the launches (C->solves); false: one of them
+// cannot be placed on the device.
 template <typename T>
-int build_solve(hf_case *C, std::vector<solve::Packed<T>> &K, const std::vector<const solve::HostSolve *> &F, SInst<T> *&dev)
+bool plan_solve(hf_case *C, const std::vector<solve::Packed<T>> &K, const std::vector<const solve::HostSolve *> &F,
+                std::vector<int> &order)
 {
     const int ni = C->ninst;
-    std::vector<int> order(ni);
+    order.resize(ni);
     for (int i = 0; i < ni; i++) order[i] = i;
     auto rows = [&](int i) { return C->coff[i + 1] - C->coff[i]; };
     auto key = [&](int i) {
@@ -2010,6 +2062,27 @@ int build_solve(hf_case *C, std::vector<solve::Packed<T>> &K, const std::vector<
         if (key(a) != key(b)) return key(a) > key(b);
         return rows(a) > rows(b);
     });
+    for (int k = 0; k < ni;) {
+        const solve::HostSolve &f = *F[order[k]];
+        int e = k;
+        size_t most = 0;
+        for (; e < ni && key(order[e]) == key(order[k]); e++) most = std::max(most, K[order[e]].smem);
+        const ClusterLaunch L(e - k, f.cluster, f.threads, most, C->stream);
+        if (!L.fits((const void *)solve_kernel<T>(f.fine, f.threads), kSolveSmem)) {
+            C->solves.clear();
+            return false;
+        }
+        C->solves.push_back(hf_case::SolveLaunch{k, e - k, f.cluster, f.fine, f.threads, most});
+        k = e;
+    }
+    return true;
+}
+
+template <typename T>
+int build_solve(hf_case *C, std::vector<solve::Packed<T>> &K, const std::vector<const solve::HostSolve *> &F,
+                const std::vector<int> &order, SInst<T> *&dev)
+{
+    const int ni = C->ninst;
     Arena ar;
     struct Where {
         size_t tables, rank_tables, ranks, rng;
@@ -2036,17 +2109,6 @@ int build_solve(hf_case *C, std::vector<solve::Packed<T>> &K, const std::vector<
     int rc = upload(C->owned, &dev, I.data(), I.size(), C->bytes, C->stream);
     if (rc) return rc;
     HF_CK(cudaStreamSynchronize(C->stream));   // the host copies go away with this function
-    for (int k = 0; k < ni;) {
-        const solve::HostSolve &f = *F[order[k]];
-        int e = k;
-        size_t most = 0;
-        for (; e < ni && key(order[e]) == key(order[k]); e++) most = std::max(most, K[order[e]].smem);
-        C->solves.push_back(hf_case::SolveLaunch{k, e - k, f.cluster, f.fine, f.threads, most});
-        auto *kern = solve_kernel<T>(f.fine, f.threads);
-        HF_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSolveSmem));
-        HF_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-        k = e;
-    }
     for (size_t k = 1; k < C->solves.size(); k++) {
         cudaStream_t st = nullptr;
         HF_CK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
@@ -2116,7 +2178,7 @@ int build_pcg(hf_case *C, const std::vector<int32_t> &mptr, const std::vector<in
         }
     }
     // the one-launch solve, when every instance's operators fit its encoding
-    // and no instance is beyond the size one cluster is the better choice for.
+    // and the device has room for its clusters.
     // Not with semi-implicit velocities: their BiCGStab solves turn a last-bit
     // change of the pressure into a change of the size of their own tolerance
     // (measured on a 96 x 96 case at rtol 1e-10: 2e-10 of u and 5e-9 of p after
@@ -2145,6 +2207,10 @@ int build_pcg(hf_case *C, const std::vector<int32_t> &mptr, const std::vector<in
         for (auto &t : th) t.join();
         fused = all;
     }
+    std::vector<const solve::HostSolve *> SF(ni);
+    std::vector<int> solve_order;
+    for (int i = 0; i < ni; i++) SF[i] = &IH[i].F;
+    if (fused) fused = mixed ? plan_solve<float>(C, K32, SF, solve_order) : plan_solve<double>(C, K64, SF, solve_order);
     C->fused = fused;
     // A case beyond that runs the level-synchronous loop on the folded
     // operators; the semi-implicit form and BiCGStab's preconditioner keep the
@@ -2480,14 +2546,13 @@ int build_pcg(hf_case *C, const std::vector<int32_t> &mptr, const std::vector<in
         C->pb32 = (float *)(base + o_pb32);
     }
     if (fused) {
-        std::vector<const solve::HostSolve *> F(ni);
         for (int i = 0; i < ni; i++) {
-            F[i] = &IH[i].F;
             const int64_t cn = IH[i].H[clev[i]].A.n;
             C->coarse_rows += cn;
             C->coarse_dense += cn * cn;
         }
-        const int rc = mixed ? build_solve<float>(C, K32, F, C->si32) : build_solve<double>(C, K64, F, C->si64);
+        const int rc = mixed ? build_solve<float>(C, K32, SF, solve_order, C->si32)
+                             : build_solve<double>(C, K64, SF, solve_order, C->si64);
         if (rc) return rc;
     }
     if (amg && !fused) {
@@ -2675,26 +2740,14 @@ void enqueue_body(hf_case *C, cudaStream_t st, cudaGraphConditionalHandle cond, 
 int enqueue_solve(hf_case *C, cudaStream_t st, int &kernels)
 {
     auto launch = [&](const hf_case::SolveLaunch &L, cudaStream_t on, bool early) -> cudaError_t {
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((unsigned)(L.count * L.cluster));
-        cfg.blockDim = dim3((unsigned)L.threads);
-        cfg.dynamicSmemBytes = L.smem;
-        cfg.stream = on;
-        cudaLaunchAttribute attr[2];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = (unsigned)L.cluster;
-        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-        // programmatic launch behind k_pcg_init, which it follows on this stream
-        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[1].val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = early ? 2 : 1;
+        ClusterLaunch K(L.count, L.cluster, L.threads, L.smem, on);
+        if (early) K.early();   // behind k_pcg_init
         kernels++;
         const PcgFine &G = C->G;
         if (C->mixed)
-            return cudaLaunchKernelEx(&cfg, solve_kernel<float>(L.fine, L.threads), G,
+            return cudaLaunchKernelEx(&K.cfg, solve_kernel<float>(L.fine, L.threads), G,
                                       SolveArgs<float>{C->si32, G.r32, C->pa32, G.e32, L.first}, L.fine);
-        return cudaLaunchKernelEx(&cfg, solve_kernel<double>(L.fine, L.threads), G,
+        return cudaLaunchKernelEx(&K.cfg, solve_kernel<double>(L.fine, L.threads), G,
                                   SolveArgs<double>{C->si64, G.r, C->pa, nullptr, L.first}, L.fine);
     };
     if (C->solves.size() > 1) HF_CK(cudaEventRecord(C->solve_events[0], st));
@@ -2779,18 +2832,8 @@ int sie_solves(hf_case *C, int64_t &launches)
                                                              C->P.sie_bc2[d], C->P.sie_b[d]);
                     launches++;
                 }
-            cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3((unsigned)(D * C->bi_cluster));
-            cfg.blockDim = dim3((unsigned)C->bi_threads[stage]);
-            cfg.dynamicSmemBytes = (size_t)C->bi_launch_smem[stage];
-            cfg.stream = st;
-            cudaLaunchAttribute attr[1];
-            attr[0].id = cudaLaunchAttributeClusterDimension;
-            attr[0].val.clusterDim.x = (unsigned)C->bi_cluster;
-            attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-            cfg.attrs = attr;
-            cfg.numAttrs = 1;
-            HF_CK(cudaLaunchKernelEx(&cfg, k_bi_solve, C->bi_args[stage]));
+            const ClusterLaunch L(D, C->bi_cluster, C->bi_threads[stage], (size_t)C->bi_launch_smem[stage], st);
+            HF_CK(cudaLaunchKernelEx(&L.cfg, k_bi_solve, C->bi_args[stage]));
             launches++;
             HF_CK(cudaMemcpyAsync(C->h_bi_sc.data(), C->bi_sc, sizeof(Scal) * D, cudaMemcpyDeviceToHost, st));
             HF_CK(cudaStreamSynchronize(st));
@@ -3947,18 +3990,24 @@ extern "C" int hf_case_create(const hf_program *pg, const hf_options *opt_in, hf
         UP(&V.sh, (const double *)nullptr, maxnf);
         UP(&V.partials, (const double *)nullptr, (size_t)blocks(maxnf) * 4);
         UP(&V.sc, (const Scal *)nullptr, 1);
-        // the one-launch form, when every system fits a cluster
+        // the one-launch form, when every system fits a cluster that the device
+        // has room for
         const int stages = C->bdf2 ? 2 : 1;
         bool fit = true;
-        for (int stage = 0; stage < stages; stage++)
-            for (int d = 0; d < D; d++) fit = fit && bi_packed[stage][d].ok;
+        C->bi_cluster = bi_packed[0][0].cluster;
+        for (int stage = 0; stage < stages; stage++) {
+            for (int d = 0; d < D; d++) {
+                const bicg::Packed &q = bi_packed[stage][d];
+                fit = fit && q.ok;
+                C->bi_threads[stage] = std::max(C->bi_threads[stage], q.threads);
+                C->bi_launch_smem[stage] = std::max(C->bi_launch_smem[stage], (int)q.smem);
+            }
+            fit = fit && ClusterLaunch(D, C->bi_cluster, C->bi_threads[stage], (size_t)C->bi_launch_smem[stage], C->stream)
+                             .fits((const void *)k_bi_solve, kBiSmem);
+        }
         if (fit) {
-            C->bi_cluster = bi_packed[0][0].cluster;
             C->h_bi_sc.resize(D);
             UP(&C->bi_sc, (const Scal *)nullptr, D);
-            if (cudaFuncSetAttribute(k_bi_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, kBiSmem) != cudaSuccess ||
-                cudaFuncSetAttribute(k_bi_solve, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
-                return cleanup(fail(HF_ERR_CUDA, "velocity solve attributes"));
             for (int stage = 0; stage < stages; stage++) {
                 BiArgs a{};
                 a.rtol = opt.poisson_rtol;
@@ -3975,8 +4024,6 @@ extern "C" int hf_case_create(const hf_program *pg, const hf_options *opt_in, hf
                     const double *x0 = stage == 0 ? F.u[d] : C->ua[d];
                     a.s[d] = BiSys{Mu.n, q.m, q.k, q.in_smem, q.ext, q.rank_bytes, mat, rng, Mu.dinv, P.sie_b[d], x0, x,
                                    C->bi_sc + d};
-                    C->bi_threads[stage] = std::max(C->bi_threads[stage], q.threads);
-                    C->bi_launch_smem[stage] = std::max(C->bi_launch_smem[stage], (int)q.smem);
                 }
                 BiArgs *dev = nullptr;
                 UP(&dev, &a, 1);
