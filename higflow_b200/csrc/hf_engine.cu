@@ -2028,11 +2028,6 @@ VLev<T> make_level(char *base, const LevelOff &o, const LevelHost &h, const TRow
     return v;
 }
 
-// Instances of up to this many rows are solved by one cluster each
-// (hf_solve.cuh); a case with a larger one runs the level-synchronous kernels,
-// which spread over the whole device.
-constexpr int kSolveMaxRows = 1 << 19;
-
 // The one-launch solves' tables of every instance on the device, the instances
 // grouped by cluster size (one launch each), largest first.
 template <typename T>
@@ -2137,10 +2132,30 @@ int build_pcg(hf_case *C, const std::vector<int32_t> &mptr, const std::vector<in
     };
     std::vector<InstHier> IH(ni);
     std::vector<int> clev(ni, 0);
+    // the one-launch solve, when every instance's operators fit its encoding
+    // and the device has room for its clusters.
+    // Not with semi-implicit velocities: their BiCGStab solves turn a last-bit
+    // change of the pressure into a change of the size of their own tolerance
+    // (measured on a 96 x 96 case at rtol 1e-10: 2e-10 of u and 5e-9 of p after
+    // one step), so that form keeps the arithmetic of the level-synchronous
+    // kernels.
+    // Its tables are encoded beside the hierarchies, the largest instance first:
+    // one that does not fit ends the encoding of the others, and where the row
+    // count alone shows that, none starts (creating 512 x 512 mixed: 1,060 ms
+    // with the encoding done for nothing, 990 without; 470 x 450 885 and 765).
+    std::vector<int> by_size(ni);
+    for (int i = 0; i < ni; i++) by_size[i] = i;
+    std::stable_sort(by_size.begin(), by_size.end(),
+                     [&](int a, int b) { return C->coff[a + 1] - C->coff[a] > C->coff[b + 1] - C->coff[b]; });
+    std::atomic<bool> fit{C->use_cg && amg && !C->sie &&
+                          C->coff[by_size[0] + 1] - C->coff[by_size[0]] <= (mixed ? solve::most_rows<float>() : solve::most_rows<double>())};
+    std::vector<solve::Packed<double>> K64(mixed ? 0 : ni);
+    std::vector<solve::Packed<float>> K32(mixed ? ni : 0);
     if (amg) {
         std::atomic<int> next{0};
         auto work = [&]() {
-            for (int i; (i = next++) < ni;) {
+            for (int k; (k = next++) < ni;) {
+                const int i = by_size[k];
                 InstHier &ih = IH[i];
                 const int c0 = C->coff[i], n = C->coff[i + 1] - c0;
                 hf::HostCSR A;
@@ -2164,40 +2179,11 @@ int build_pcg(hf_case *C, const std::vector<int32_t> &mptr, const std::vector<in
                 std::vector<double> inv;
                 if (!hf::dense_inverse(last.A, inv)) { ih.err = "singular coarsest AMG level"; continue; }
                 ih.inv = std::move(inv);
-                if (C->use_cg && !C->sie && n <= kSolveMaxRows) ih.F = solve::build(ih.H, ih.inv, C->P.ncell);
-            }
-        };
-        const unsigned nt = std::max(1u, std::min(std::thread::hardware_concurrency(), 32u));
-        std::vector<std::thread> th;
-        for (unsigned t = 0; t + 1 < nt && (int)t < ni; t++) th.emplace_back(work);
-        work();
-        for (auto &t : th) t.join();
-        for (int i = 0; i < ni; i++) {
-            if (!IH[i].err.empty()) return fail(HF_ERR_UNSUPPORTED, IH[i].err + " (instance " + std::to_string(i) + ")");
-            clev[i] = (int)IH[i].H.size() - 1;
-        }
-    }
-    // the one-launch solve, when every instance's operators fit its encoding
-    // and the device has room for its clusters.
-    // Not with semi-implicit velocities: their BiCGStab solves turn a last-bit
-    // change of the pressure into a change of the size of their own tolerance
-    // (measured on a 96 x 96 case at rtol 1e-10: 2e-10 of u and 5e-9 of p after
-    // one step), so that form keeps the arithmetic of the level-synchronous
-    // kernels.
-    bool fused = C->use_cg && amg && !C->sie;
-    for (int i = 0; i < ni && fused; i++) fused = IH[i].F.ok;
-    std::vector<solve::Packed<double>> K64;
-    std::vector<solve::Packed<float>> K32;
-    if (fused) {
-        if (mixed) K32.resize(ni);
-        else K64.resize(ni);
-        std::atomic<int> next{0};
-        std::atomic<bool> all{true};
-        auto work = [&]() {
-            for (int i; (i = next++) < ni;) {
-                if (mixed) K32[i] = solve::pack<float>(IH[i].F, IH[i].inv, true);
-                else K64[i] = solve::pack<double>(IH[i].F, IH[i].inv, false);
-                if (!(mixed ? K32[i].ok : K64[i].ok)) all = false;
+                if (!fit) continue;
+                ih.F = solve::build(ih.H, ih.inv, C->P.ncell);
+                if (ih.F.ok && mixed) K32[i] = solve::pack<float>(ih.F, ih.inv, true);
+                else if (ih.F.ok) K64[i] = solve::pack<double>(ih.F, ih.inv, false);
+                if (!ih.F.ok || !(mixed ? K32[i].ok : K64[i].ok)) fit = false;
             }
         };
         const unsigned nt = std::max(1u, std::min(std::thread::hardware_concurrency(), 32u));
@@ -2205,8 +2191,12 @@ int build_pcg(hf_case *C, const std::vector<int32_t> &mptr, const std::vector<in
         for (unsigned t = 0; t + 1 < nt && (int)t + 1 < ni; t++) th.emplace_back(work);
         work();
         for (auto &t : th) t.join();
-        fused = all;
+        for (int i = 0; i < ni; i++) {
+            if (!IH[i].err.empty()) return fail(HF_ERR_UNSUPPORTED, IH[i].err + " (instance " + std::to_string(i) + ")");
+            clev[i] = (int)IH[i].H.size() - 1;
+        }
     }
+    bool fused = fit;
     std::vector<const solve::HostSolve *> SF(ni);
     std::vector<int> solve_order;
     for (int i = 0; i < ni; i++) SF[i] = &IH[i].F;

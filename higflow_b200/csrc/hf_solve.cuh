@@ -1082,6 +1082,16 @@ inline HostSolve build(const std::vector<hf::HostLevel> &H, const std::vector<do
     return S;
 }
 
+// Rows beyond which an instance fits no cluster: r, q, z and the row descriptors
+// always lie in shared memory (with halos, coarse levels and operators beside
+// them 73,000 rows of a square fit in FP64 and 130,000 in FP32, of these 109,000
+// and 174,000)
+template <typename T>
+constexpr int most_rows()
+{
+    return kSolveMaxCluster * (kSolveSmem / (3 * (int)sizeof(T) + (int)sizeof(uint2)));
+}
+
 // the instance's tables and its shared-memory layout
 template <typename T>
 struct Packed {
