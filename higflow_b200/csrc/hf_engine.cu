@@ -2143,6 +2143,8 @@ int build_pcg(hf_case *C, const std::vector<int32_t> &mptr, const std::vector<in
     // one that does not fit ends the encoding of the others, and where the row
     // count alone shows that, none starts (creating 512 x 512 mixed: 1,060 ms
     // with the encoding done for nothing, 990 without; 470 x 450 885 and 765).
+    int sms = 0;
+    HF_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, C->opt.device));
     std::vector<int> by_size(ni);
     for (int i = 0; i < ni; i++) by_size[i] = i;
     std::stable_sort(by_size.begin(), by_size.end(),
@@ -2180,7 +2182,7 @@ int build_pcg(hf_case *C, const std::vector<int32_t> &mptr, const std::vector<in
                 if (!hf::dense_inverse(last.A, inv)) { ih.err = "singular coarsest AMG level"; continue; }
                 ih.inv = std::move(inv);
                 if (!fit) continue;
-                ih.F = solve::build(ih.H, ih.inv, C->P.ncell);
+                ih.F = solve::build(ih.H, ih.inv, C->P.ncell, sms);
                 if (ih.F.ok && mixed) K32[i] = solve::pack<float>(ih.F, ih.inv, true);
                 else if (ih.F.ok) K64[i] = solve::pack<double>(ih.F, ih.inv, false);
                 if (!ih.F.ok || !(mixed ? K32[i].ok : K64[i].ok)) fit = false;

@@ -861,10 +861,10 @@ struct HostSolve {
 // 128 cavities of 2.06 M rows in all, whole step: 2.65 ms, 3.75 at 512 rows
 // whatever the batch.  The sums' grouping, so the last bits, follow the batch.
 constexpr int kSolveRows = 512;
-inline int cluster_size(int n, long total)
+inline int cluster_size(int n, long total, int sms)
 {
     int rows = kSolveRows;
-    while (rows < 4096 && total > 148l * rows) rows *= 2;
+    while (rows < 4096 && total > (long)sms * rows) rows *= 2;
     int c = 1;
     while (c < kSolveMaxCluster && (long)c * rows < n) c *= 2;
     return c;
@@ -993,13 +993,13 @@ inline void coarse_operator(HostSolve &S, const std::vector<double> &inverse)
     S.cpos.clear();
 }
 
-inline HostSolve build(const std::vector<hf::HostLevel> &H, const std::vector<double> &inverse, long total)
+inline HostSolve build(const std::vector<hf::HostLevel> &H, const std::vector<double> &inverse, long total, int sms)
 {
     HostSolve S;
     S.clev = (int)H.size() - 1;
     S.nc = H.back().A.n;
     if (S.nc > kCoarseCap || S.clev >= kMaxLevels) return S;
-    S.cluster = S.clev == 0 ? 1 : cluster_size(H[0].A.n, total);
+    S.cluster = S.clev == 0 ? 1 : cluster_size(H[0].A.n, total, sms);
     S.threads = block_threads((H[0].A.n + S.cluster - 1) / S.cluster, total > H[0].A.n);
     S.L.resize(std::max(1, S.clev));
     for (int l = 0; l < (int)S.L.size(); l++) {
