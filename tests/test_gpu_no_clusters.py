@@ -16,6 +16,7 @@ import sys
 
 import numpy as np
 import pytest
+import torch
 
 from higflow_b200 import engine
 from higflow_b200 import program as hp
@@ -28,7 +29,8 @@ cases = importlib.util.module_from_spec(_spec)
 _spec.loader.exec_module(cases)
 
 EXPLICIT = [("9x9", "plain"), ("33x31", "plain"), ("33x31", "mixed"), ("9x10x9", "plain"), ("9,40,20", "mixed")]
-BOXES = ["6x5", "33x32", "96x96", "128x129", "9x8x10"]
+BOXES = ["6x5", "33x32", "96x96", "128x129", "180x180", "9x8x10"]
+RESIDUALS = ["33x31", "129x128", "240x200", "17x16x17"]
 GOLDEN = ["sie2d_cubista", "cn2d_cubista", "bdf2_cav2d", "bdf2_cav3d", "bdf2_oldroyd_log", "cn2d_oldroyd_log",
           "sie2d_oldroyd_log", "amr2d_sie_oldroyd"]
 
@@ -48,6 +50,33 @@ def _run(case):
     out["loop"], out["launches"] = c.launch_counts()[1], c.stats().kernel_launches
     c.close()
     return out
+
+
+def _residual_run(sides):
+    """One step at Poisson rtol 1e-15: (dp, u*)."""
+    case = _box(sides)
+    c = engine.Case(cases._programs(case)[0], engine.options(rtol=1e-15, atol=1e-300))
+    for k, v in cases._inputs(case, 7)[1].items():
+        c.set(*k, v)
+    c.step(1)
+    out = c.get(hp.FIELD_DP), [c.get(hp.FIELD_USTAR, d) for d in range(c.prog.dim)]
+    c.close()
+    return out
+
+
+def _true_residual(sides, dp, us):
+    """||b - A dp|| / ||b|| over the rows beside the pinned one, A dp in extended
+    precision."""
+    case = _box(sides)
+    prog, shape = cases._programs(case)[0], cases._shapes(case)[0]
+    ex = cases._Exact(prog, shape, "cpu")
+    u = [torch.as_tensor(x) for x in us]
+    b = sum(ex.q(ex.ds[2 * d + 1], u[d]) - ex.q(ex.ds[2 * d], u[d]) for d in range(prog.dim)).numpy() / ex.h / prog.par["dt"]
+    row = np.repeat(np.arange(prog.ncell), np.diff(prog.p_ptr))
+    r = b.astype(np.longdouble)
+    np.subtract.at(r, row, np.asarray(prog.p_val).astype(np.longdouble) * dp.astype(np.longdouble)[prog.p_col])
+    r[prog.pin_row] = 0
+    return float(np.sqrt((r * r).sum()) / np.linalg.norm(b))
 
 
 def _run_golden(name):
@@ -90,6 +119,20 @@ def test_explicit_steps_run_on_the_launch_loop(without_clusters, sides, precisio
         assert err < (1e-10 if precision == "plain" else 1e-6), (k, err)
 
 
+@pytest.mark.parametrize("sides", RESIDUALS)
+def test_the_one_launch_solve_attains_the_loops_residual(without_clusters, sides):
+    """The one-launch solve carries q = A z + beta q where the loop multiplies A p
+    anew.  Plain solves driven to where ||r|| of the recurrence reaches 1e-15:
+    what is left of b - A x itself may be 4 times the loop's (the errors of
+    earlier products enter q's with weights beta, beta^2, ...: 1 / (1 - beta) of
+    the loop's, beta up to 0.7)."""
+    dp, us = _residual_run(sides)
+    ours = _true_residual(sides, dp, us)
+    loops = _true_residual(sides, without_clusters[f"{sides}/residual/dp"],
+                           [without_clusters[f"{sides}/residual/u{d}"] for d in range(len(us))])
+    assert 0.0 < ours <= 4.0 * loops, (ours, loops)
+
+
 @pytest.mark.parametrize("sides", BOXES)
 def test_semi_implicit_boxes_keep_their_bits(without_clusters, sides):
     _same_bits(_run(_box(sides, scheme="semi_implicit")), without_clusters, f"{sides}/sie/")
@@ -104,6 +147,10 @@ def _child(out):
     fields = {}
     for sides, precision in EXPLICIT:
         fields.update({f"{sides}/{precision}/{k}": v for k, v in _run(_box(sides, precision)).items()})
+    for sides in RESIDUALS:
+        dp, us = _residual_run(sides)
+        fields.update({f"{sides}/residual/u{d}": v for d, v in enumerate(us)})
+        fields[f"{sides}/residual/dp"] = dp
     for sides in BOXES:
         fields.update({f"{sides}/sie/{k}": v for k, v in _run(_box(sides, scheme="semi_implicit")).items()})
     for name in GOLDEN:
