@@ -16,9 +16,13 @@ between chunks of steps, when its cohort's stream is idle.  A request whose
 step fails (a NaN, a Poisson solve that does not converge) is frozen by the
 engine at that step and fails alone; the rest of its cohort goes on.
 
-Each instance's reductions are deterministic and per instance (see
-hf_pcg.cuh), so a request's result does not depend on the other requests of
-its cohort: the same alone and in any mix (tests/test_gpu_serve.py).
+A request's result agrees with its run alone to the Poisson solves' tolerance
+(within 1e-10 relative L2 at Poisson rtol 1e-13: tests/test_gpu_serve.py,
+tests/test_gpu_alone_and_batched.py), not to the bit: each instance's reductions
+are its own and deterministic, but how its rows are split over SMs, and with
+that the order of its sums, follows the cohort's size (hf_solve.cuh), and beside
+an instance too large for one cluster it runs on the launch loop's kernels.  The
+same cohort gives the same bits every time.
 
 No counterpart in the reference, which runs one case per job.
 """

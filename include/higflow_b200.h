@@ -378,9 +378,12 @@ int  hf_case_set_timestep(hf_case *c, const double *dt, int32_t n);
 /* Per-instance step limits (no counterpart in the reference, which runs one
  * case per job): instance i takes steps[i] more steps and is then frozen (no
  * kernel changes its fields) while the others go on; steps[i] < 0: no limit.
- * n = ninst.  Each frozen instance's fields stay those of its last step, so
- * its result is the same as when it runs alone for steps[i] steps.  Needs the
- * CG Poisson path and an explicit velocity scheme (HF_ERR_UNSUPPORTED
+ * n = ninst.  Each frozen instance's fields stay those of its last step: those
+ * of steps[i] steps alone, to the Poisson solves' tolerance (a batch groups an
+ * instance's sums otherwise, and runs it on other kernels beside an instance too
+ * large for one cluster: within 1e-10 relative L2 at poisson_rtol 1e-13, not the
+ * same bits).  The same batch gives the same bits every time.  Needs the CG
+ * Poisson path and an explicit velocity scheme (HF_ERR_UNSUPPORTED
  * otherwise).  Once limits are set, an instance whose step fails (a NaN, a
  * Poisson solve that does not converge) is frozen after that step and the
  * others go on; the step call still returns the first failure. */
