@@ -167,8 +167,13 @@ class ClockSampler:
 # ---------------------------------------------------------------------------
 # algorithmic bytes per step of each phase (higflow_b200/roofline.py: the
 # reference's kernels' field arrays plus the stencil bytes of their distinct
-# queries; the Poisson iterations at the measured count)
-def phase_bytes(prog, mixed, iters_per_step, sweeps_per_step):
+# queries; the Poisson iterations at the measured count).  one_launch: the solve
+# runs as one launch that keeps its vectors on the chip (k_solve), so the phase
+# moves the operator and each vector once per step (the residual, the initial
+# guess and the unknown's history in, the unknown and its history out; mixed: the
+# FP32 residual too, and per sweep the FP64 residual and unknown both ways),
+# whatever the iterations
+def phase_bytes(prog, mixed, iters_per_step, sweeps_per_step, one_launch=False):
     from higflow_b200 import roofline
     sb = roofline.step_bytes(prog, mixed)
     nc = prog.ncell
@@ -181,6 +186,9 @@ def phase_bytes(prog, mixed, iters_per_step, sweeps_per_step):
            "poisson_iter": iters_per_step * roofline.poisson_iter_bytes(prog, 4 if mixed else 8)
            + sweeps_per_step * spmv64,
            "final": sb["final"]["F"] + sb["final"]["S"]}
+    if one_launch:
+        out["poisson_iter"] = (4 * (nc + 1) + prog.p_col.size * (4 + w) + 8 * 7 * nc
+                               + ((4 + sweeps_per_step * 8 * 4) * nc if mixed else 0))
     if "ve_cell" in sb:
         out["ve_cell"] = sb["ve_cell"]["F"] + sb["ve_cell"]["S"]
         # k_ve_cell alone: the stage without the polymeric tensor (k_ve_stress
@@ -473,6 +481,7 @@ def run_b200(args, rank, world, device):
     iters = st.total_iters - st0.total_iters
     phases = case.phase_times()
     shapes = dict(zip(("k_vrows", "k_velocity", "k_ve_cell"), case.launch_shapes()))
+    one_launch = case.launch_counts()[1] == 0
     case.profile(False)
     t_s = _max_over_ranks(dev_ms / 1e3, world, device)
     value = cells * args.steps * world / t_s
@@ -483,7 +492,7 @@ def run_b200(args, rank, world, device):
     sizes = np.diff(prog.cell_off) if prog.ninst > 1 else np.array([prog.ncell])
     it_step = float((dit * sizes).sum()) / float(sizes.sum()) / args.steps
     sweeps = float(st.last_outer) if mixed else 0.0
-    pb, sb = phase_bytes(prog, mixed, it_step, sweeps)
+    pb, sb = phase_bytes(prog, mixed, it_step, sweeps, one_launch)
     peak, peak_kind = _peaks()
     phase_rl = {}
     for p, (ms, nl) in phases.items():
@@ -592,6 +601,7 @@ def run_b200(args, rank, world, device):
                      "peak_source": peak_kind + " (MEASURED_PEAKS.json hbm_gbs)" if peak_kind == "measured" else peak_kind},
         "whole_step_roofline": whole,
         "phase_roofline": phase_rl,
+        "poisson_one_launch": one_launch,
         "e2e": e2e,
         "gpu_launches": int(launches),
         "poisson_iters_per_step": iters / args.steps,

@@ -343,8 +343,9 @@ int  hf_case_solver_info(hf_case *c, int32_t *method, int32_t *nlev, int64_t *ro
  * kernel (k_velocity), [2] cell stage (k_ve_cell); n >= 3. */
 int  hf_case_launch_shapes(hf_case *c, int32_t *blocks, int32_t n);
 
-/* Kernels per step outside the Poisson iterations, and per loop body of the
- * iterations (one body = two CG iterations). */
+/* Kernels per step outside the Poisson loop, and per loop body (one body = two
+ * CG iterations).  Where the solve runs as one launch per cluster size there is
+ * no loop: per_body is 0 and those launches count in per_step. */
 int  hf_case_launch_counts(hf_case *c, int32_t *per_step, int32_t *per_body);
 
 /* Batches: number of instances, and the last step's Poisson result of one
