@@ -110,6 +110,7 @@ __device__ __forceinline__ void team_sum(Team &t, double (&tot)[NV])
 
 }  // namespace bicg
 
+// (64 registers a thread at 1,024 threads; ptxas spills 16 bytes beyond them)
 __global__ void __launch_bounds__(kBiThreads, 1) k_bi_solve(const BiArgs *args)
 {
     using bicg::at;

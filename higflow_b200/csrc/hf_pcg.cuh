@@ -738,7 +738,9 @@ __global__ void __launch_bounds__(kBlock) k_vf_down(VLev<T> L, VLev<T> Ln, const
 template <typename T, typename Fn>
 __device__ __forceinline__ void folded_up(const VLev<T> &L, const pcg::RowSet &R, const T *e, T (&s)[kRPT], Fn b)
 {
-    // (a row's entries eight at a time: their loads are in flight together)
+    // (unrolled by eight, so that the loads of several entries are in flight: as
+    // many as the 32 registers a thread that ptxas takes here can hold, fewer than
+    // eight in FP64, where k_vf_z spills 36 bytes)
 #pragma unroll
     for (int q = 0; q < kRPT; q++) {
         s[q] = T(0);

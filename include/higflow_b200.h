@@ -302,7 +302,8 @@ typedef struct hf_stats {
     int32_t last_iters;       /* Poisson iterations of the last step (inner)   */
     int32_t last_outer;       /* refinement sweeps of the last step (mixed:    */
                               /* the most of any instance; plain: 1)           */
-    double  last_residual;    /* relative true residual of the last solve      */
+    double  last_residual;    /* relative residual of the last solve (mixed:   */
+                              /* of b - A x; plain: of the CG recurrence)     */
     int64_t total_iters;      /* all Poisson iterations since create           */
     int64_t kernel_launches;  /* kernels launched by hf_case_step so far       */
     double  device_bytes;     /* HBM held by this case                         */
